@@ -477,6 +477,9 @@ void build_params(StepParams<A>& P, const ch4_config& c, const Lattice& lat, con
   P.zfirst = 0;
   P.zstride = 1;
   P.zcount = c.NZ;
+  P.zcells = (uint32_t)N;
+  P.div_nx = fast_div_of((uint32_t)c.NX);
+  P.div_nxy = fast_div_of((uint32_t)c.NX * (uint32_t)c.NY);
   P.Lhit = c.NX + c.NY + (c.nz_global > 0 ? c.nz_global : c.NZ);
   uint32_t F = 0;
   const uint64_t fl = c.flags;

@@ -94,15 +94,38 @@ enum : uint32_t {
   W_SZ = 1u << 13        // scalar walls on z
 };
 
+// n / d for 0 <= n < 2^31 as a multiplication: with l = ceil(log2 d) >= 1 and
+// mul = floor(2^(31 + l) / d) + 1 < 2^32, n * mul / 2^(31 + l) exceeds n / d by less than
+// n / 2^(31 + l) < 1/d (Granlund and Montgomery 1994); d = 1 is passed through
+struct FastDiv {
+  uint32_t mul, shift, one;
+};
+inline FastDiv fast_div_of(uint32_t d) {
+  if (d <= 1) return {0u, 0u, 1u};
+  uint32_t l = 1;
+  while (l < 31 && (1u << l) < d) l++;
+  return {(uint32_t)(((1ull << (31 + l)) / d) + 1ull), l - 1, 0u};
+}
+__host__ __device__ __forceinline__ uint32_t fast_div(uint32_t n, const FastDiv& d) {
+#ifdef __CUDA_ARCH__
+  const uint32_t hi = __umulhi(n, d.mul);
+#else
+  const uint32_t hi = (uint32_t)(((uint64_t)n * d.mul) >> 32);
+#endif
+  return d.one ? n : hi >> d.shift;
+}
+
 template <typename A>
 struct StepParams {
   int NX, NY, NZ;
   long long N;  // cells
+  FastDiv div_nx, div_nxy;  // by NX and NX * NY
   int zoff;     // global z of plane 0 (z-slab of a larger lattice), else 0
   // planes of one launch of the step kernel: zfirst + k * zstride, k < zcount (the whole
   // lattice: 0, 1, NZ; a slab that overlaps its face exchange steps its two face planes
   // and then its interior)
   int zfirst, zstride, zcount;
+  uint32_t zcells;  // NX * NY * zcount
   int Lhit;     // NX + NY + global NZ: length of one HIT table row
   uint32_t feat;
   uint32_t walls;  // W_* bits
@@ -175,17 +198,24 @@ struct Codec;
 
 template <>
 struct Codec<double, double> {
+  static constexpr bool deviation = false;
   __device__ __forceinline__ static double load(const double* p, long long i, double, double) { return __ldg(p + i); }
   __device__ __forceinline__ static void store(double* p, long long i, double v, double, double) { p[i] = v; }
 };
 template <>
 struct Codec<float, float> {
+  static constexpr bool deviation = false;
+  __device__ __forceinline__ static float load_raw(const float* p, long long i) { return __ldg(p + i); }
+  __device__ __forceinline__ static void store_raw(float* p, long long i, float v) { p[i] = v; }
   __device__ __forceinline__ static float load(const float* p, long long i, float, float) { return __ldg(p + i); }
   __device__ __forceinline__ static void store(float* p, long long i, float v, float, float) { p[i] = v; }
 };
 // IEEE half holding the deviation f_q - w_q * shift
 template <>
 struct Codec<__half, float> {
+  static constexpr bool deviation = true;
+  __device__ __forceinline__ static float load_raw(const __half* p, long long i) { return __half2float(__ldg(p + i)); }
+  __device__ __forceinline__ static void store_raw(__half* p, long long i, float v) { p[i] = __float2half_rn(v); }
   __device__ __forceinline__ static float load(const __half* p, long long i, float w, float shift) {
     return __half2float(__ldg(p + i)) + w * shift;
   }

@@ -71,12 +71,6 @@ __device__ __forceinline__ A cdot_rt(int q, A ux, A uy, A uz) {
 }
 
 // (c - u) * invcs2 + c * cu * invcs4 for one component (src/forcing.c:1427-1429)
-template <int cc, typename A>
-__device__ __forceinline__ A guo_d(A u, A cu, A invcs2, A invcs4) {
-  if constexpr (cc == 0) return (-u) * invcs2;
-  else if constexpr (cc > 0) return (A(1) - u) * invcs2 + cu * invcs4;
-  else return (A(-1) - u) * invcs2 + (-cu) * invcs4;
-}
 template <typename A>
 __device__ __forceinline__ A guo_d_rt(int cc, A u, A cu, A invcs2, A invcs4) {
   if (cc == 0) return (-u) * invcs2;

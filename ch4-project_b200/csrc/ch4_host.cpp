@@ -683,6 +683,9 @@ struct Engine : EngineBase {
   double* pf_alt = nullptr;
   int* pid_alt = nullptr;
   int since_reorder = 0;
+  // the state planes whose values differ between particles (or may, once the kernels write
+  // them): the only ones that a re-sort has to move
+  PartPlanes planes{};
   // z-slab particles: set_particles / get_particles take every particle of the lattice
   // (np_all); the slab holds np of them.  The particles' u has two halo planes on either
   // side; particles that leave the slab move through four buffers (send down, send up,
@@ -711,9 +714,11 @@ struct Engine : EngineBase {
   int* mig_cnt = nullptr;
   size_t uplane() const { return (size_t)c.NX * c.NY * 4; }  // values of one plane of upart
   A* ut_in() const { return upart + (pslab() ? 2 * uplane() : 0); }
-  // re-sort of the state slots by home cell every REORDER_EVERY steps (a particle
-  // moves well under a cell in that time, so the order stays close to sorted)
-  static constexpr int REORDER_EVERY = 4;
+  // re-sort of the state slots by home row every REORDER_EVERY steps (a particle moves a cell
+  // or two in that time, so neighbours stay neighbours).  us a step every 4 / 8 / 16 steps:
+  // 40,000 tracers in 96^3 LES 75.3 / 66.0 / 61.3, 250,000 two-way in 160^3 438 / 433 / 431
+  static constexpr int REORDER_EVERY = 16;
+  bool upart_current = false;  // upart holds u^n of the populations as they are
   A* upart = nullptr;     // (u_x, u_y, u_z, t)^{n+1} per cell for the interpolation
   A* dbuf[2] = {nullptr, nullptr};  // two-way deposit of this / previous step
   int dcur_i = 0;
@@ -722,6 +727,8 @@ struct Engine : EngineBase {
   double* rec = nullptr;
   double* srec = nullptr;
   int* spid = nullptr;
+  int* row_start = nullptr;  // list starts of the deposit by rows
+  bool rows_ready = false;   // its records and keys are those of the state (the last sub-step wrote them)
   int2* crng = nullptr;   // {start, end} per home cell
   int* busy = nullptr;    // cells for the deposit merge pass, per gather block
   int *bcount = nullptr, *boff = nullptr, *dense = nullptr;
@@ -783,6 +790,7 @@ struct Engine : EngineBase {
     cudaFree(dbuf[0]);
     cudaFree(dbuf[1]);
     cudaFree(crng);
+    cudaFree(row_start);
     cudaFree(busy);
     cudaFree(bcount);
     cudaFree(boff);
@@ -837,7 +845,11 @@ struct Engine : EngineBase {
   bool twoway_temp() const { return (c.flags2 & CH4_F2_LAGRANGE_TWOWAY_TEMPERATURE) != 0; }
   // deposit record fields: fac*fp (3) + the stencil weights (6 trilinear, 12 tricubic), then
   // with the thermal coupling fac*sp
-  int nrec() const { return ((c.flags & CH4_F_LAGRANGE_TWOWAY_TRICUBIC) ? 15 : 9) + (twoway_temp() ? 1 : 0); }
+  // the plain trilinear momentum deposit of a whole lattice goes by rows (deposit_rows.cuh)
+  bool by_rows() const {
+    return twoway() && !twoway_temp() && !pslab() && !(c.flags & CH4_F_LAGRANGE_TWOWAY_TRICUBIC);
+  }
+  int nrec() const { return by_rows() ? ROW_REC : ((c.flags & CH4_F_LAGRANGE_TWOWAY_TRICUBIC) ? 15 : 9) + (twoway_temp() ? 1 : 0); }
   // planes of a deposit buffer: the force, and the temperature source with the thermal coupling
   int dplanes() const { return twoway_temp() ? 4 : 3; }
 
@@ -897,6 +909,9 @@ struct Engine : EngineBase {
                : (c.flags2 & CH4_F2_LAGRANGE_ORIENTATION_ACTIVE_SELECTIVEORIENTATION) ? 5
                                                                                     : 1;
     Q.nrec = nrec();
+    Q.rows = by_rows();
+    Q.row_start = row_start;
+    Q.rows_ready = rows_ready;
     Q.rec = rec;
     Q.srec = srec;
     Q.spid = spid;
@@ -1029,11 +1044,38 @@ struct Engine : EngineBase {
     return st;
   }
 
+  void find_planes(const std::vector<double>& h, size_t n) {
+    const uint64_t fl = c.flags, f2 = c.flags2;
+    auto in = [](int f, int lo, int hi) { return f >= lo && f <= hi; };
+    auto written = [&](int f) {
+      if (pslab()) return true;  // the exchange moves whole records
+      if (in(f, CH4_PF(x), CH4_PF(uz_old))) return true;  // x, v, a, u and their old values
+      if (in(f, CH4_PF(dx_ux), CH4_PF(dz_uz))) return (fl & CH4_F_LAGRANGE_GRADIENT) != 0;
+      if (in(f, CH4_PF(Dt_ux), CH4_PF(Dt_uz))) return (fl & CH4_F_LAGRANGE_ADDEDMASS) != 0;
+      if (in(f, CH4_PF(t), CH4_PF(dz_t))) return nsets_on[1] != 0;
+      if (f == CH4_PF(t_p)) return (f2 & CH4_F2_LAGRANGE_TEMPERATURE) != 0;
+      if (f == CH4_PF(sediment)) return (f2 & CH4_F2_LAGRANGE_BC_INELASTIC_SEDIMENT) != 0;
+      // orientations, swimming and jump state
+      if (in(f, CH4_PF(px), CH4_PF(dt_pz)) || in(f, CH4_PF(nx), CH4_PF(dt_nz)) ||
+          in(f, CH4_PF(shear_rate), CH4_PF(pz_jump)))
+        return (fl & CH4_F_LAGRANGE_ORIENTATION) != 0;
+      return false;
+    };
+    planes.n = 0;
+    for (int f = 0; f < PF_TOTAL; f++) {
+      const double* v = h.data() + (size_t)f * n;
+      bool move = written(f);
+      if (!move && n > 1) move = std::memcmp(v, v + 1, (n - 1) * sizeof(double)) != 0;  // each equals its neighbour
+      if (move) planes.f[planes.n++] = (unsigned char)f;
+    }
+  }
+
   ch4_status set_particles(const ch4_particle* parts, int n) override {
     if (!lagr()) return H->fail(CH4_ERR_ARG, "particles need the LAGRANGE flag");
     if (n < 0 || (n > 0 && !parts)) return H->fail(CH4_ERR_ARG, "bad particle array");
     ch4_status st;
     if ((st = H->cuda(cudaStreamSynchronize(H->stream), "sync"))) return st;
+    rows_ready = false;
     const bool sl = pslab();
     if (n != (sl ? np_all : np) || (sl && !mig)) {
       free_particles();
@@ -1048,8 +1090,8 @@ struct Engine : EngineBase {
                     cudaMalloc(&key2, sizeof(unsigned) * n) == cudaSuccess &&
                     cudaMalloc(&order, sizeof(int) * n) == cudaSuccess &&
                     cudaMalloc(&order2, sizeof(int) * n) == cudaSuccess &&
-                    (!twoway() || (cudaMalloc(&rec, sizeof(double) * nrec() * (size_t)n) == cudaSuccess &&
-                                   cudaMalloc(&srec, sizeof(double) * nrec() * (size_t)n) == cudaSuccess &&
+                    (!twoway() || cudaMalloc(&rec, sizeof(double) * nrec() * (size_t)n) == cudaSuccess) &&
+                    (!twoway() || (cudaMalloc(&srec, sizeof(double) * nrec() * (size_t)n) == cudaSuccess &&
                                    cudaMalloc(&spid, sizeof(int) * (size_t)n) == cudaSuccess));
           if (!ok) return H->fail(CH4_ERR_NOMEM, "sort buffers");
           if (rj_random() && (cudaMalloc(&rj_count, sizeof(int) * (size_t)n) != cudaSuccess ||
@@ -1113,8 +1155,10 @@ struct Engine : EngineBase {
       }
     }
     if (n > 0 &&
-        (st = H->cuda(cudaMemcpy(pf, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice), "particles up")))
+        ((st = H->cuda(cudaMemcpy(pf, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice), "particles up")) ||
+         (st = H->cuda(cudaMemcpy(pf_alt, pf, sizeof(double) * h.size(), cudaMemcpyDeviceToDevice), "particles up"))))
       return st;
+    find_planes(h, n);
     since_reorder = REORDER_EVERY;  // sort at the first opportunity
     if (n == 0) return CH4_OK;
     return H->cuda(cudaMemcpy(pid, ids.data(), sizeof(int) * n, cudaMemcpyHostToDevice), "particle ids up");
@@ -1228,7 +1272,8 @@ struct Engine : EngineBase {
   ch4_status reorder_particles(int sort) {
     PartParams<A> Q = part_params();
     size_t bytes = cubbytes;
-    ch4_status st = H->cuda(launch_particle_reorder(Q, key2, order2, cubtmp, bytes, sort, H->stream), "reorder");
+    ch4_status st =
+        H->cuda(launch_particle_reorder(Q, planes, key2, order2, cubtmp, bytes, sort, H->stream), "reorder");
     if (st) return st;
     std::swap(pf, pf_alt);
     std::swap(pid, pid_alt);
@@ -1380,7 +1425,10 @@ struct Engine : EngineBase {
           return H->fail(CH4_ERR_CUDA, "deposit memset");
       }
       const size_t nreg = (size_t)((c.NX + GATHER_BLOCK - 1) / GATHER_BLOCK) * c.NY * c.NZ;
-      if (cudaMalloc(&crng, sizeof(int2) * nhome()) != cudaSuccess ||
+      if (by_rows()) {
+        if (cudaMalloc(&row_start, sizeof(int) * ((size_t)row_bins(c.NX, c.NY, c.NZ) + 1)) != cudaSuccess)
+          return H->fail(CH4_ERR_NOMEM, "row lists");
+      } else if (cudaMalloc(&crng, sizeof(int2) * nhome()) != cudaSuccess ||
           cudaMalloc(&busy, sizeof(int) * nreg * GATHER_BLOCK) != cudaSuccess ||
           cudaMalloc(&dense, sizeof(int) * nreg * GATHER_BLOCK) != cudaSuccess ||
           cudaMalloc(&bcount, sizeof(int) * nreg) != cudaSuccess || cudaMalloc(&boff, sizeof(int) * nreg) != cudaSuccess)
@@ -1554,6 +1602,7 @@ struct Engine : EngineBase {
   }
 
   ch4_status set_pop(int set, const double* aos, int brd) override {
+    upart_current = false;
     if (!nsets_on[set]) return H->fail(CH4_ERR_ARG, "population set %d is not enabled", set);
     H->initialized = false;
     rest_pending[set] = false;
@@ -1637,6 +1686,7 @@ struct Engine : EngineBase {
   }
 
   ch4_status initialize() override {
+    upart_current = false;
     if (ch4_status rs = ready()) return rs;
     bind_pops(cur);
     ch4_status st;
@@ -1831,8 +1881,12 @@ struct Engine : EngineBase {
           P.fm_cur = fmbuf + 6 * (fm_i ^ 1);
           if ((st = force_moments(P.hit_cur, 1, fmbuf + 6 * (fm_i ^ 1)))) return st;
         }
-        if (c.flags & CH4_F_FLUID_LES)
-          if ((st = les_u())) return st;
+        if (c.flags & CH4_F_FLUID_LES) {
+          // with particles u^n is at hand: the vectors the last step interpolated (the same
+          // hydro pass with the same force), a pass of 15 us in 96^3 FP32
+          P.ules = upart_current ? upart : ules;
+          if (!upart_current && (st = les_u())) return st;
+        }
         if (sism()) {  // this step's running mean of u, from the last one and u^n
           P.um_old = um_a;
           P.um_new = um_b;
@@ -1857,12 +1911,15 @@ struct Engine : EngineBase {
                                          nullptr, nullptr, nullptr, H->stream, ut_in()),
                             "particle u")))
             return st;
+          upart_current = c.nz_global <= 0;
           if (pslab() && (st = u_halo())) return st;
           for (int sub = 0; sub < (int)c.time_dt_lagr_factor; sub++) {
             if (noise() && np > 0 && (st = draw_noise())) return st;
             PartParams<A> Q = part_params();
             Q.first = (n_step == 1 && c.resume == 0);
             Q.time_now = H->time_now;
+            Q.emit = by_rows() && !rj_random() && sub + 1 == (int)c.time_dt_lagr_factor;
+            rows_ready = Q.emit != 0;
             if ((st = H->cuda(launch_particle_substep(Q, H->stream), "particle substep"))) return st;
             if (rj_random() && np > 0 && (st = reinject_random())) return st;
             if (pslab() && (st = migrate())) return st;  // move_particles ends with sendrecv_particles

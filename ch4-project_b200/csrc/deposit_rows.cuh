@@ -1,0 +1,252 @@
+// Two-way momentum deposit by lattice rows (included by particles.cuh inside namespace ch4).
+//
+// src/lagrange_feedback.c:11-256: the particle loop adds fac * fp * vol of every particle to
+// the 8 cells of its stencil.  Here the particles are radix-sorted (stably, laid out by
+// particle index) by the row segment their home cell lies in -- at most ROW_SEG cells of one
+// (y, z) row -- and one warp owns one segment of a lattice row: it merges the lists of the
+// four home rows around it in particle-index order and adds every particle to the two cells
+// it has in the row, in shared memory.  Each cell thus sums its particles in the reference's
+// order whatever the schedule, and no array runs over the home cells.
+//
+// Why rows: at the workloads' 0.04 depositing particles per cell nearly every home cell is
+// empty, and a list per home cell (a range of 8 bytes each, cleared, filled, read and scanned
+// every step) moved more bytes than the particles; a row of 256 cells has some 10 particles a
+// list.  Keys are 8-10 bits shorter too, one to two radix passes less, and the records and keys
+// are written by the sub-step that has their inputs in registers.  Measured, us a step: 250,000
+// particles in 160^3 FP32 505 -> 431, 15,000 in 60x50x70 FP64 164 -> 109 (re-sort every 16 steps
+// and only of the planes that differ included).
+#pragma once
+
+constexpr int ROW_SEG = 256;    // cells of a row that one warp owns
+constexpr int ROW_CHUNK = 64;   // merged entries in shared memory at a time (8 lists x 8)
+constexpr int ROW_WARPS = 4;    // warps per block
+constexpr int ROW_REC = 10;     // doubles of a record: fac*fp (3), dxm dxp dym dyp dzm dzp, {hx, index}
+
+// row segments along x: the last home cell (hx = NX) belongs to the last segment
+__host__ __device__ __forceinline__ int row_segs(int NX) { return (NX + ROW_SEG - 1) / ROW_SEG; }
+__host__ __device__ __forceinline__ unsigned int row_bins(int NX, int NY, int NZ) {
+  return (unsigned)row_segs(NX) * (unsigned)(NY + 1) * (unsigned)(NZ + 1);
+}
+__host__ __device__ __forceinline__ unsigned int row_bin(int hx, int hy, int hz, int NX, int NY) {
+  const int ns = row_segs(NX), s = hx / ROW_SEG;
+  return ((unsigned)hz * (unsigned)(NY + 1) + (unsigned)hy) * (unsigned)ns + (unsigned)(s < ns ? s : ns - 1);
+}
+
+#ifdef __CUDACC__
+
+// Deposit record and row-segment key of one particle (src/lagrange_feedback.c:34-118).  The
+// last sub-step of a step calls it with the state it has in registers; a and D (acceleration
+// and Du/Dt) are read from the state where `have` is not set.
+template <typename A>
+__device__ __forceinline__ void deposit_rows_emit(const PartParams<A>& P, int ip, double x, double y, double z,
+                                                  double beta, bool have, const double* a, const double* D) {
+  const double* pf = P.pf;
+  const long long np = P.np;
+#define F(name) pf[CH4_PF(name) * np + ip]
+  Stencil t;
+  double px, py, pz;
+  const bool inside = wrapped_position(P, x, y, z, px, py, pz);
+  make_stencil(px, py, pz, t);
+  const double fac = pf[PF_VOL * np + ip];
+  const int o = P.pid[ip];
+  const bool live = inside && (fac > 0.0) && beta != 0.0;
+  const int hx = t.im + 1, hy = t.jm + 1, hz = t.km + 1;
+  const unsigned int nb = row_bins(P.NX, P.NY, P.NZ);
+  P.key[o] = (live ? 0u : nb) + row_bin(hx, hy, hz, P.NX, P.NY);
+  P.order[o] = ip;
+  if (!live) return;  // sorted after every list and never read
+  const double dr = pf[PF_DR * np + ip];
+  double aa[3], DD[3];
+  if (have) {
+#pragma unroll
+    for (int q = 0; q < 3; q++) aa[q] = a[q], DD[q] = D[q];
+  } else {
+    aa[0] = F(ax), aa[1] = F(ay), aa[2] = F(az);
+    DD[0] = F(Dt_ux), DD[1] = F(Dt_uy), DD[2] = F(Dt_uz);
+  }
+#undef F
+  // gravity_vector of src/lagrange_feedback.c:95-103 (y points down)
+  const double g[3] = {P.gravity ? P.g[0] : 0.0, P.gravity ? -P.g[1] : 0.0, P.gravity ? P.g[2] : 0.0};
+  double f[3];
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    if (P.twoway_stau) f[q] = fac * ((DD[q] - g[q]) * (1 - dr));  // src/lagrange_feedback.c:106-110
+    else f[q] = fac * (DD[q] - g[q] + dr * (g[q] - aa[q]));
+  }
+  double2* r = reinterpret_cast<double2*>(P.rec + (long long)ip * ROW_REC);
+  r[0] = make_double2(f[0], f[1]);
+  r[1] = make_double2(f[2], t.dxm);
+  r[2] = make_double2(t.dxp, t.dym);
+  r[3] = make_double2(t.dyp, t.dzm);
+  r[4] = make_double2(t.dzp, __hiloint2double(o, hx));
+}
+
+// the same from the state (a resumed run's first deposit; random re-entry, which moves
+// particles after the sub-step)
+template <typename A>
+__global__ void deposit_rows_prepare_kernel(const PartParams<A> P) {
+  const int ip = blockIdx.x * blockDim.x + threadIdx.x;
+  if (ip >= P.np) return;
+  const long long np = P.np;
+  deposit_rows_emit(P, ip, P.pf[CH4_PF(x) * np + ip], P.pf[CH4_PF(y) * np + ip], P.pf[CH4_PF(z) * np + ip],
+                    P.pf[CH4_PF(beta_coeff) * np + ip], false, (const double*)nullptr, (const double*)nullptr);
+}
+
+// The records of the depositing particles in sorted order (a list is then one run of them: no
+// load of the merge waits for an index), and start[b] = first sorted position with a key of at
+// least b, b = 0 .. nb; the blocks from `copies` on do the second.
+static __global__ void row_lists_kernel(const unsigned int* __restrict__ key, const int* __restrict__ slot, int n,
+                                        unsigned int nb, int copies, const double2* __restrict__ rec, double2* srec,
+                                        int* start) {
+  if ((int)blockIdx.x < copies) {
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const int i = (int)(t / (ROW_REC / 2)), part = (int)(t % (ROW_REC / 2));
+    if (i < n && key[i] < nb) srec[t] = rec[(long long)slot[i] * (ROW_REC / 2) + part];
+    return;
+  }
+  const unsigned int b = (blockIdx.x - (unsigned)copies) * blockDim.x + threadIdx.x;
+  if (b > nb) return;
+  int lo = 0, hi = n;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (key[mid] < b) lo = mid + 1;
+    else hi = mid;
+  }
+  start[b] = lo;
+}
+
+// shared memory of one warp: the contributions by merged position (component c of corner di
+// at 2 c + di), the row's sums (three rows of `cells`), indices and cells of the merged entries
+__host__ __device__ __forceinline__ int row_cells(int NX) { return NX < ROW_SEG ? (NX + 1) & ~1 : ROW_SEG; }
+__host__ __device__ __forceinline__ int row_shared(int NX) {
+  return ROW_CHUNK * 6 * 8 + 3 * row_cells(NX) * 8 + ROW_CHUNK * 2 * 4;
+}
+
+template <typename A>
+__global__ void __launch_bounds__(32 * ROW_WARPS) deposit_rows_kernel(const PartParams<A> P) {
+  extern __shared__ double row_smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cells = row_cells(P.NX);
+  double* const con = row_smem + warp * (row_shared(P.NX) / 8);
+  double* const acc = con + ROW_CHUNK * 6;
+  int* const s_pid = reinterpret_cast<int*>(acc + 3 * cells);
+  int* const s_x = s_pid + ROW_CHUNK;
+  const int ns = row_segs(P.NX);
+  const long long w = (long long)blockIdx.x * ROW_WARPS + warp;
+  if (w >= (long long)ns * P.NY * P.NZ) return;  // whole warps: no block barrier below
+  const int seg = (int)(w % ns), j = (int)((w / ns) % P.NY), k = (int)(w / ((long long)ns * P.NY));
+  const int x0 = seg * ROW_SEG, n = min(ROW_SEG, P.NX - x0);
+  A* out = P.dep + ((long long)k * P.NY + j) * P.NX + x0;
+  // lane l < 4: the home row (y + (l & 1), z + (l >> 1)) of this segment; 4 <= l < 8: the same
+  // rows' next segment, whose first home cell also deposits into this one's last cell
+  int beg = 0, end = 0;
+  if (lane < 8 && (lane < 4 || seg + 1 < ns)) {
+    const unsigned int b = ((unsigned)(k + ((lane >> 1) & 1)) * (unsigned)(P.NY + 1) + (unsigned)(j + (lane & 1))) *
+                               (unsigned)ns + (unsigned)(seg + (lane >> 2));
+    beg = P.row_start[b];
+    end = P.row_start[b + 1];
+  }
+  constexpr unsigned ALL = 0xffffffffu;
+  if (__any_sync(ALL, beg < end)) {
+    for (int c = lane; c < n; c += 32) acc[c] = acc[cells + c] = acc[2 * cells + c] = 0.0;
+    // chunks of the merge: up to cap entries of each list; with entries left behind, only those
+    // up to the smallest index T that ends a cut list are merged now
+    while (__any_sync(ALL, beg < end)) {
+      const int left = __reduce_add_sync(ALL, end - beg);
+      const int cap = left <= ROW_CHUNK ? ROW_CHUNK : ROW_CHUNK / (ns == 1 ? 4 : 8);
+      const int cnt = min(end - beg, cap);
+      int off = cnt;  // inclusive prefix over the lists, then exclusive
+#pragma unroll
+      for (int d = 1; d < 8; d <<= 1) {
+        const int v = __shfl_up_sync(ALL, off, d);
+        if (lane >= d && lane < 8) off += v;
+      }
+      const int total = __shfl_sync(ALL, off, 7);
+      off -= cnt;
+      for (int e = lane; e < ROW_CHUNK; e += 32) {
+        const bool on = e < total;
+        int l = 0;
+#pragma unroll
+        for (int q = 1; q < 8; q++)  // the last list that begins at or before e
+          if (__shfl_sync(ALL, off, q) <= e) l = q;
+        const int base = __shfl_sync(ALL, beg, l) - __shfl_sync(ALL, off, l);
+        if (on) s_pid[e] = __double2hiint(P.srec[(long long)(base + e) * ROW_REC + 9]);
+      }
+      __syncwarp();
+      const bool cut = lane < 8 && end - beg > cnt;
+      const int T = __reduce_min_sync(ALL, cut ? s_pid[off + cnt - 1] : 0x7fffffff);
+      for (int e = lane; e < ROW_CHUNK; e += 32) {
+        const int pid = e < total ? s_pid[e] : 0x7fffffff;
+        const bool on = e < total && pid <= T;
+        int rank = 0, l = 0;
+#pragma unroll
+        for (int q = 0; q < 8; q++) {  // entries of list q below this one (its own: its position)
+          const int a = __shfl_sync(ALL, off, q), c = __shfl_sync(ALL, cnt, q);
+          if (a <= e) l = q;
+          if (!on) continue;
+          int lo = 0, hi = c;
+          while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (s_pid[a + mid] < pid) lo = mid + 1;
+            else hi = mid;
+          }
+          rank += lo;
+        }
+        const int base = __shfl_sync(ALL, beg, l) - __shfl_sync(ALL, off, l);
+        if (on) {
+          const double2* r = reinterpret_cast<const double2*>(P.srec + (long long)(base + e) * ROW_REC);
+          const double2 a = r[0], b = r[1], c = r[2], d = r[3], f = r[4];
+          const double wy = (l & 1) ? d.x : c.y;         // dyp : dym
+          const double wz = ((l >> 1) & 1) ? f.x : d.y;  // dzp : dzm
+          const double v0 = b.y * wy * wz, v1 = c.x * wy * wz;
+          double* o = con + 6 * rank;
+          o[0] = a.x * v0;
+          o[1] = a.x * v1;
+          o[2] = a.y * v0;
+          o[3] = a.y * v1;
+          o[4] = b.x * v0;
+          o[5] = b.x * v1;
+          s_x[rank] = __double2loint(f.y) - x0;
+        }
+      }
+      // how many entries of each list were merged: those up to T
+      int done = cnt;
+      if (lane < 8) {
+        int lo = 0, hi = cnt;
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (s_pid[off + mid] <= T) lo = mid + 1;
+          else hi = mid;
+        }
+        done = lo;
+      }
+      const int merged = __reduce_add_sync(ALL, lane < 8 ? done : 0);
+      __syncwarp();
+      // in particle order: lane 2 c + di adds component c to the corner di of the stencil
+      for (int e0 = 0; e0 < merged; e0 += 4) {
+        int cell[4];
+        double v[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const int e = min(e0 + q, merged - 1);
+          cell[q] = e0 + q < merged && lane < 6 ? s_x[e] - (lane & 1) : -1;
+          v[q] = con[6 * e + (lane < 6 ? lane : 0)];
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          if (cell[q] >= 0 && cell[q] < n) acc[(lane >> 1) * cells + cell[q]] += v[q];
+          __syncwarp();
+        }
+      }
+      beg += done;
+    }
+    for (int c = lane; c < n; c += 32) {
+      out[c] = (A)acc[c];
+      out[P.N + c] = (A)acc[cells + c];
+      out[2 * P.N + c] = (A)acc[2 * cells + c];
+    }
+  } else {
+    for (int c = lane; c < n; c += 32) out[c] = out[P.N + c] = out[2 * P.N + c] = A(0);
+  }
+}
+
+#endif  // __CUDACC__

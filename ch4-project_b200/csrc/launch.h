@@ -72,9 +72,9 @@ cudaError_t launch_halo_copy(const HaloCopy& H, cudaStream_t st);
 
 // Lagrangian particles: state slot i <- slot order2[i] into P.pf_alt / P.pid_alt (with
 // sort != 0 the home-cell keys are computed and radix-sorted into key2 / order2 first)
-cudaError_t launch_particle_reorder(const PartParams<double>& P, unsigned int* key2, int* order2, void* tmp,
+cudaError_t launch_particle_reorder(const PartParams<double>& P, const PartPlanes& planes, unsigned int* key2, int* order2, void* tmp,
                                     size_t& tmp_bytes, int sort, cudaStream_t st);
-cudaError_t launch_particle_reorder(const PartParams<float>& P, unsigned int* key2, int* order2, void* tmp,
+cudaError_t launch_particle_reorder(const PartParams<float>& P, const PartPlanes& planes, unsigned int* key2, int* order2, void* tmp,
                                     size_t& tmp_bytes, int sort, cudaStream_t st);
 // Lagrangian particles: one sub-step (interpolate + move + wrap)
 cudaError_t launch_particle_substep(const PartParams<double>& P, cudaStream_t st);

@@ -439,11 +439,11 @@ __device__ __forceinline__ void hydro_cell(const StepParams<A>& P, int x, int y,
 template <typename S, typename A, bool THERM, bool SCAL>
 __global__ void hydro_kernel(const StepParams<A> P, const A* hit, const A* dep, const A* fm, double* dens, double* u,
                              double* t, double* s, double* force, A* u_arith, A* ut4, int ut4_t) {
-  // grid (x blocks, NY, NZ): no index division
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= P.NX) return;
-  const int y = blockIdx.y, z = blockIdx.z;
-  const long long idx = ((long long)z * P.NY + y) * P.NX + x;
+  // one thread per cell whatever NX is, as the step kernel
+  const unsigned int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= P.zcells) return;
+  const unsigned int k = fast_div(idx, P.div_nxy), r = idx - k * (unsigned)(P.NX * P.NY);
+  const int y = (int)fast_div(r, P.div_nx), x = (int)r - y * P.NX, z = (int)k;
   A rho, ux, uy, uz, Fx, Fy, Fz;
   hydro_cell<S, A, THERM, SCAL>(P, x, y, z, idx, hit, dep, fm, rho, ux, uy, uz, Fx, Fy, Fz);
   if (dens) dens[idx] = (double)rho;

@@ -43,6 +43,12 @@ constexpr int PF_TOTAL = PF_FIELDS + 4;
 constexpr int GATHER_BLOCK = 128;  // threads (cells along x) per block of the first deposit pass
 constexpr int GATHER_KB = 8;       // planes per block of that pass (each thread walks a column)
 
+// the state planes that a re-sort of the slots moves (the others hold one value each)
+struct PartPlanes {
+  int n;
+  unsigned char f[PF_TOTAL];
+};
+
 template <typename A>
 struct PartParams {
   int NX, NY, NZ;
@@ -77,6 +83,12 @@ struct PartParams {
   int nrec;              // fields of a record: 9 (trilinear) or 15 (tricubic)
   double* rec;           // [nrec][np] per state slot: fac*fp (3), then dxm dxp dym dyp dzm dzp
                          // (trilinear) or the cubic weights wx[4] wy[4] wz[4] (tricubic)
+  // trilinear momentum deposit by lattice rows (deposit_rows.cuh): rec then holds ROW_REC
+  // doubles per state slot, one record after the other
+  int rows;
+  int rows_ready;        // the last sub-step wrote the records and keys
+  int emit;              // this sub-step writes them
+  int* row_start;        // [row_bins + 1] first sorted position of every row segment's list
   double* srec;          // [nrec][np] the same by sorted position (depositing particles only)
   int* spid;             // particle index by sorted position
   int2* cell_rng;        // [(NX+1)(NY+1)(NZ+1)] {start, end} of every home cell's sorted run
@@ -807,6 +819,10 @@ static __device__ __noinline__ void swim_velocity(double* pf, long long np, int 
 #undef F
 }
 
+template <typename A>
+__device__ __forceinline__ void deposit_rows_emit(const PartParams<A>& P, int ip, double x, double y, double z,
+                                                  double beta, bool have, const double* a, const double* D);
+
 // One Lagrangian sub-step for one particle: interpolate, move, wrap.  The state the
 // step reads is loaded once, up front (independent loads), and every result is
 // stored once at the end; the arithmetic is the reference's, expression for
@@ -945,6 +961,8 @@ __global__ void __launch_bounds__(128, sizeof(A) == 8 ? 2 : 4) particle_substep_
   // gravity_coeff; 1 without LAGRANGE_GRAVITY_VARIABLE, where c g and (-beta) c g equal g and
   // (-beta) g exactly
   const double gc = P.gravity_var ? F(gravity_coeff) : 1.0;
+  double dep_a[3], dep_D[3];  // for the deposit record, where this sub-step forms both
+  bool dep_have = false;
   if (tau > 0.0) {  // Stokes drag (+ added mass)
     const double invtau = 1.0 / tau;
     double ax = (ux - vx) * invtau, ay = (uy - vy) * invtau, az = (uz - vz) * invtau;
@@ -1008,6 +1026,11 @@ __global__ void __launch_bounds__(128, sizeof(A) == 8 ? 2 : 4) particle_substep_
       vy += dtl * 0.5 * (3.0 * ay - F(ay_old));
       vz += dtl * 0.5 * (3.0 * az - F(az_old));
     }
+    if (P.addedmass && beta != 0.0) {
+      dep_have = true;
+      dep_a[0] = ax, dep_a[1] = ay, dep_a[2] = az;
+      dep_D[0] = Dx, dep_D[1] = Dy, dep_D[2] = Dz;
+    }
     F(ax) = ax;
     F(ay) = ay;
     F(az) = az;
@@ -1064,10 +1087,14 @@ __global__ void __launch_bounds__(128, sizeof(A) == 8 ? 2 : 4) particle_substep_
     F(t_p) = (tp + fac1 * v[NF - 1]) * e;
   }
   // ---- LAGRANGE_WRAP of sendrecv_particles
-  F(x) = pwrapd(xn, P.SX);
-  F(z) = pwrapd(zn, P.SZ);
-  F(y) = pwrapd(yn, P.SY);
+  xn = pwrapd(xn, P.SX);
+  yn = pwrapd(yn, P.SY);
+  zn = pwrapd(zn, P.SZ);
+  F(x) = xn;
+  F(z) = zn;
+  F(y) = yn;
 #undef F
+  if (P.emit) deposit_rows_emit(P, ip, xn, yn, zn, beta, dep_have, dep_a, dep_D);
 }
 
 // Keys cubic kernel of the tricubic deposit (src/lagrange_feedback.c:839-848)
@@ -1151,16 +1178,18 @@ __global__ void particle_key_kernel(const PartParams<A> P) {
   P.order[o] = ip;
 }
 
-// slot i of (pf_alt, pid_alt) <- slot src[i] of (pf, pid)
+// slot i of (pf_alt, pid_alt) <- slot src[i] of (pf, pid), for the planes that differ between
+// particles (pf_alt holds the others since the upload).  HBM-bound: 16 bytes a plane and
+// particle; of the 75 planes a two-way run without orientation or temperature moves 40.
 template <typename A>
-__global__ void particle_permute_kernel(const PartParams<A> P, const int* __restrict__ src) {
+__global__ void particle_permute_kernel(const PartParams<A> P, const PartPlanes L, const int* __restrict__ src) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= P.np) return;
   const long long np = P.np;
   const int s = src[i];
   P.pid_alt[i] = P.pid[s];
 #pragma unroll 5
-  for (int f = 0; f < PF_TOTAL; f++) P.pf_alt[f * np + i] = P.pf[f * np + s];
+  for (int q = 0; q < L.n; q++) P.pf_alt[L.f[q] * np + i] = P.pf[L.f[q] * np + s];
 }
 
 // z-slab particle exchange (sendrecv_particles, src/lagrange.c:4028-4221).  A particle
@@ -1607,4 +1636,7 @@ __global__ void deposit_tricubic_kernel(const PartParams<A> P) {
 }
 
 #endif  // __CUDACC__
+
+#include "deposit_rows.cuh"
+
 }  // namespace ch4

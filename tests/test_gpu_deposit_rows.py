@@ -1,0 +1,72 @@
+"""The two-way deposit by lattice rows (csrc/deposit_rows.cuh) where its lists are unusual:
+rows of two and three segments (particles at the segment ends included), lists longer than
+the chunk that a warp merges at a time, runs that re-sort the slots, a particle count that
+leaves most lists empty, and uploads in the middle of a run.  FP64, bit-identical to the
+restatement; FP32 the same from call to call."""
+import numpy as np
+import pytest
+
+import oracle as O
+from lbcases import make_case, make_particles, run_restatement
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("no CUDA device", allow_module_level=True)
+
+import ch4b200  # noqa: E402
+
+
+def small_particles(rng, n, size, box, at=None):
+    """Inertial particles (radius small against a cell) and tracers in the corner `box`."""
+    parts = make_particles(rng, n, *size)
+    for i, p in enumerate(parts):
+        p.tau_drag = [0.8, 0.0, 1.5, 1.0][i % 4]
+        p.beta_coeff = [1.0, 0.5, 0.0][i % 3]
+        p.x, p.y, p.z = (rng.random() * b for b in box)
+        if at and i % 3 == 0:  # about the homes at a segment's end
+            p.x = at[i % len(at)] + 0.9 * (rng.random() - 0.5)
+    return parts
+
+
+CASES = {
+    "segments": dict(dims=(530, 3, 3), n=700, box=(530, 3, 3), at=(255.5, 256.5, 511.5, 512.5, 0.3, 529.7), steps=6),
+    "dense": dict(dims=(10, 8, 7), n=600, box=(2, 2, 2), at=None, steps=3),
+    "dense_segments": dict(dims=(300, 4, 3), n=500, box=(300, 2, 2), at=(255.6, 256.2), steps=3),
+    "sparse": dict(dims=(40, 9, 8), n=5, box=(40, 9, 8), at=None, steps=10),
+}
+
+
+def run(cfg, state, parts, steps):
+    with ch4b200.Simulation(cfg) as sim:
+        sim.set_pop("p", state["p"])
+        sim.set_particles(parts)
+        sim.initialize()
+        sim.step(1)
+        sim.set_particles(sim.get_particles(len(parts)))  # the state as it is, re-uploaded
+        sim.step(steps - 1)
+        return sim.get_pop("p"), O.particles_as_dict(sim.get_particles(len(parts)))
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_rows_bit_identical(name):
+    c = CASES[name]
+    _, cfg, state = make_case("particles", seed=2, dims=c["dims"])
+    parts = small_particles(np.random.default_rng(7), c["n"], c["dims"], c["box"], c["at"])
+    ref = run_restatement(cfg, dict(state, part=parts), c["steps"])
+    assert np.isfinite(ref["p"]).all()
+    p, got = run(cfg, state, parts, c["steps"])
+    assert np.array_equal(p, ref["p"])
+    for k, v in ref["part"].items():
+        assert np.array_equal(got[k], v), k
+
+
+@pytest.mark.parametrize("name", ["segments", "dense"])
+def test_rows_f32_reproducible(name):
+    c = CASES[name]
+    _, cfg, state = make_case("particles", seed=2, dims=c["dims"], storage=1)
+    parts = small_particles(np.random.default_rng(7), c["n"], c["dims"], c["box"], c["at"])
+    a, b = run(cfg, state, parts, c["steps"]), run(cfg, state, parts, c["steps"])
+    assert np.array_equal(a[0], b[0])
+    assert all(np.array_equal(a[1][k], b[1][k]) for k in a[1])

@@ -456,15 +456,6 @@ void normalize_averages(const ch4_config& c, const int* nsets_on, double* h) {
   }
 }
 
-// plane pointers of set s from its base pointers (N cells, `bytes` per stored value)
-template <typename A>
-void set_planes(StepParams<A>& P, int s, long long N, size_t bytes) {
-  for (int q = 0; q < NPOP; q++) {
-    P.fin_q[s][q] = P.fin[s] ? static_cast<const char*>(P.fin[s]) + (size_t)q * N * bytes : nullptr;
-    P.fout_q[s][q] = P.fout[s] ? static_cast<char*>(P.fout[s]) + (size_t)q * N * bytes : nullptr;
-  }
-}
-
 // Parameter block of one lattice from its configuration (host FP64 -> arithmetic type A).
 template <typename A>
 void build_params(StepParams<A>& P, const ch4_config& c, const Lattice& lat, const double* hit_fac, long long N,
@@ -478,6 +469,7 @@ void build_params(StepParams<A>& P, const ch4_config& c, const Lattice& lat, con
   P.zstride = 1;
   P.zcount = c.NZ;
   P.zcells = (uint32_t)N;
+  P.bstride = (uint32_t)(Q * POP_BLOCK * (1 + nsets_on[1] + nsets_on[2]));
   P.div_nx = fast_div_of((uint32_t)c.NX);
   P.div_nxy = fast_div_of((uint32_t)c.NX * (uint32_t)c.NY);
   P.Lhit = c.NX + c.NY + (c.nz_global > 0 ? c.nz_global : c.NZ);
@@ -757,9 +749,7 @@ struct Engine : EngineBase {
     shape.storage = c.storage;
   }
   ~Engine() override {
-    for (auto& s : f)
-      for (auto& b : s)
-        if (b) cudaFree(b);
+    for (void* b : f[0]) cudaFree(b);  // all sets lie in the fluid's buffers
     cudaFree(tprev);
     cudaFree(sprev);
     cudaFree(kol);
@@ -1308,38 +1298,26 @@ struct Engine : EngineBase {
   // the bottom row) has no source row: the cell's own wall rule writes it (bounce-back,
   // or the fixed-value rule of a temperature/scalar wall), not a stream from across the
   // face, so that row stays out of the exchange (a slip wall streams it: exchanged).
-  ch4_status halo(bool pack, void* a, void* b) override {
+  ch4_status halo(bool pack, void* down, void* up) override {
     if (ch4_status rs = ready()) return rs;
-    const size_t row = (size_t)c.NX * sbytes, plane = row * c.NY, top = (size_t)(c.NZ - 1) * plane;
     const uint32_t F = P.feat;
+    HaloFacesArgs a{};
+    a.NX = c.NX;
+    a.NY = c.NY;
+    a.NZ = c.NZ;
+    a.pops = f[0][cur];
+    a.down = down;
+    a.up = up;
+    a.pack = pack;
     const bool local_top[3] = {(F & K_FWALL) && !(F & K_FSLIP_P), (F & K_TWALL) != 0, (F & K_SWALL) != 0};
     const bool local_bot[3] = {(F & K_FWALL) && !(F & K_FSLIP_M), (F & K_TWALL) != 0, (F & K_SWALL) != 0};
-    HaloCopy hc{};
-    int slot = 0;
     for (int s = 0; s < 3; s++) {
       if (!nsets_on[s]) continue;
-      char* base = static_cast<char*>(f[s][cur]);
-      int kd = 0, ku = 0;
-      for (int q = 0; q < NPOP; q++) {
-        if (cz(q) == 0) continue;
-        char* qplane = base + (size_t)q * N * sbytes;
-        // c_z = -1: the top plane holds the values sent down; c_z = +1: the bottom plane those sent up
-        char* face = cz(q) < 0 ? qplane + top : qplane;
-        char* buf = static_cast<char*>(cz(q) < 0 ? a : b) + ((size_t)slot * 5 + (cz(q) < 0 ? kd++ : ku++)) * plane;
-        size_t off = 0, bytes = plane;
-        if (cy(q) < 0 && local_top[s]) bytes -= row;  // rows 0 .. NY-2
-        if (cy(q) > 0 && local_bot[s]) {              // rows 1 .. NY-1
-          off = row;
-          bytes -= row;
-        }
-        hc.src[hc.n] = (pack ? face : buf) + off;
-        hc.dst[hc.n] = (pack ? buf : face) + off;
-        hc.bytes[hc.n] = bytes;
-        hc.n++;
-      }
-      slot++;
+      if (local_top[s]) a.own |= 1u << a.sets;
+      if (local_bot[s]) a.own |= 8u << a.sets;
+      a.sets++;
     }
-    return H->cuda(launch_halo_copy(hc, H->stream), pack ? "halo pack" : "halo unpack");
+    return H->cuda(launch_halo_faces(a, sbytes, H->stream), pack ? "halo pack" : "halo unpack");
   }
 
   ch4_status particle_averages(int types, double* out) override {
@@ -1387,12 +1365,11 @@ struct Engine : EngineBase {
     return CH4_OK;
   }
 
+  int sets() const { return 1 + nsets_on[1] + nsets_on[2]; }
   int L() const { return c.NX + c.NY + H->nz_all(); }  // HIT table row: the whole lattice's z
 
   size_t device_bytes() const override {
-    size_t b = 0;
-    for (int s = 0; s < 3; s++)
-      if (nsets_on[s]) b += 2 * (size_t)NPOP * N * sbytes;
+    size_t b = 2 * pop_values(N, sets()) * sbytes;
     if (nsets_on[1]) b += N * sizeof(A);
     if (nsets_on[2]) b += N * sizeof(A);
     if (c.flags & CH4_F_FLUID_LES) b += 4 * N * sizeof(A);
@@ -1402,13 +1379,11 @@ struct Engine : EngineBase {
   }
 
   ch4_status alloc() override {
-    cudaError_t e;
-    for (int s = 0; s < 3; s++) {
-      if (!nsets_on[s]) continue;
-      for (int b = 0; b < 2; b++) {
-        e = cudaMalloc(&f[s][b], (size_t)NPOP * N * sbytes);
-        if (e != cudaSuccess) return H->fail(CH4_ERR_NOMEM, "population buffer: %s", cudaGetErrorString(e));
-      }
+    for (int b = 0; b < 2; b++) {
+      const cudaError_t e = cudaMalloc(&f[0][b], pop_values(N, sets()) * sbytes);
+      if (e != cudaSuccess) return H->fail(CH4_ERR_NOMEM, "population buffer: %s", cudaGetErrorString(e));
+      for (int s = 1, k = 1; s < 3; s++)
+        if (nsets_on[s]) f[s][b] = static_cast<char*>(f[0][b]) + (size_t)(k++) * Q * POP_BLOCK * sbytes;
     }
     if (nsets_on[1] && cudaMalloc(&tprev, N * sizeof(A)) != cudaSuccess) return H->fail(CH4_ERR_NOMEM, "tprev");
     if (nsets_on[2] && cudaMalloc(&sprev, N * sizeof(A)) != cudaSuccess) return H->fail(CH4_ERR_NOMEM, "sprev");
@@ -1533,7 +1508,6 @@ struct Engine : EngineBase {
     for (int s = 0; s < 3; s++) {
       P.fin[s] = f[s][in];
       P.fout[s] = f[s][in ^ 1];
-      set_planes(P, s, N, sbytes);
     }
   }
 
@@ -3582,7 +3556,7 @@ size_t slot_bytes(const ch4_config& c, int storage) {
   const size_t N = (size_t)c.NX * c.NY * c.NZ;
   const size_t sb = storage == CH4_STORE_F16 ? 2 : 4;
   int sets = 1 + ((c.flags & CH4_F_LB_TEMPERATURE) != 0) + ((c.flags & CH4_F_LB_SCALAR) != 0);
-  size_t b = (size_t)sets * 2 * NPOP * N * sb;
+  size_t b = 2 * pop_values((long long)N, sets) * sb;
   if (c.flags & CH4_F_LB_TEMPERATURE) b += N * 4;
   if (c.flags & CH4_F_LB_SCALAR) b += N * 4;
   b += (size_t)(2 * c.NY + c.NX) * 4;
@@ -3683,7 +3657,6 @@ struct ch4_ensemble {
     for (int k = 0; k < 3; k++) {
       P.fin[k] = s.f[k][in];
       P.fout[k] = s.f[k][in ^ 1];
-      set_planes(P, k, s.N, storage == CH4_STORE_F16 ? 2 : 4);
     }
     return P;
   }
@@ -3795,11 +3768,10 @@ ch4_status ch4_ensemble_create(int storage, size_t budget, ch4_ensemble** out) {
 }
 
 static void free_slot(Slot& s) {
-  for (auto& a : s.f)
-    for (auto& b : a) {
-      cudaFree(b);
-      b = nullptr;
-    }
+  for (int b = 0; b < 2; b++) {
+    cudaFree(s.f[0][b]);  // all sets lie in the fluid's buffers
+    s.f[0][b] = s.f[1][b] = s.f[2][b] = nullptr;
+  }
   cudaFree(s.tprev);
   cudaFree(s.sprev);
   cudaFree(s.kol);
@@ -3861,9 +3833,11 @@ ch4_status ch4_ensemble_add(ch4_ensemble* E, const ch4_config* cfg, int* slot) {
   s.nsets_on[2] = sh.scal;
   const size_t sb = E->storage == CH4_STORE_F16 ? 2 : 4;
   bool ok = true;
-  for (int k = 0; k < 3 && ok; k++)
-    if (s.nsets_on[k])
-      for (int b = 0; b < 2 && ok; b++) ok = cudaMalloc(&s.f[k][b], (size_t)NPOP * s.N * sb) == cudaSuccess;
+  for (int b = 0; b < 2 && ok; b++) {
+    ok = cudaMalloc(&s.f[0][b], pop_values(s.N, 1 + sh.therm + sh.scal) * sb) == cudaSuccess;
+    for (int k = 1, at = 1; k < 3 && ok; k++)
+      if (s.nsets_on[k]) s.f[k][b] = static_cast<char*>(s.f[0][b]) + (size_t)(at++) * Q * POP_BLOCK * sb;
+  }
   if (ok && sh.therm) ok = cudaMalloc(&s.tprev, s.N * sizeof(float)) == cudaSuccess;
   if (ok && sh.scal) ok = cudaMalloc(&s.sprev, s.N * sizeof(float)) == cudaSuccess;
   const int nk = 2 * cfg->NY + cfg->NX;

@@ -85,6 +85,7 @@ __device__ __forceinline__ void deposit_rows_emit(const PartParams<A>& P, int ip
 // particles after the sub-step)
 template <typename A>
 __global__ void deposit_rows_prepare_kernel(const PartParams<A> P) {
+  grid_chain();
   const int ip = blockIdx.x * blockDim.x + threadIdx.x;
   if (ip >= P.np) return;
   const long long np = P.np;
@@ -95,9 +96,9 @@ __global__ void deposit_rows_prepare_kernel(const PartParams<A> P) {
 // The records of the depositing particles in sorted order (a list is then one run of them: no
 // load of the merge waits for an index), and start[b] = first sorted position with a key of at
 // least b, b = 0 .. nb; the blocks from `copies` on do the second.
-static __global__ void row_lists_kernel(const unsigned int* __restrict__ key, const int* __restrict__ slot, int n,
-                                        unsigned int nb, int copies, const double2* __restrict__ rec, double2* srec,
-                                        int* start) {
+static __global__ void row_lists_kernel(const unsigned int* key, const int* slot, int n, unsigned int nb,
+                                        int copies, const double2* rec, double2* srec, int* start) {
+  grid_chain();
   if ((int)blockIdx.x < copies) {
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const int i = (int)(t / (ROW_REC / 2)), part = (int)(t % (ROW_REC / 2));
@@ -124,6 +125,7 @@ __host__ __device__ __forceinline__ int row_shared(int NX) {
 
 template <typename A>
 __global__ void __launch_bounds__(32 * ROW_WARPS) deposit_rows_kernel(const PartParams<A> P) {
+  grid_chain();
   extern __shared__ double row_smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cells = row_cells(P.NX);
   double* const con = row_smem + warp * (row_shared(P.NX) / 8);

@@ -2,8 +2,15 @@
 // the B200 lattice-Boltzmann step.
 //
 // Lattice tables: src/lb.c:139-230 (weights, velocities, opposite directions).
-// Populations live on the device as SoA planes f[q][z][y][x] (x fastest), one
-// plane per direction q, so every warp access is a contiguous row segment.
+// Populations live on the device in blocks of POP_BLOCK = 32 consecutive cells (x fastest,
+// then y, z): a block holds, for every enabled set in the order p, g, h, the 19 directions'
+// 32 values one after the other.  A warp access is then one contiguous run, as it would be
+// with one plane per direction, but all directions of a cell lie at constant distances: one
+// address serves the 19 to 57 loads of a cell and the one to three stores of a direction.
+// (With planes, half of the step kernel's instructions formed addresses: 450 of 902 per warp
+// of 32 cells, FP32 fluid and temperature.)  us a step, planes -> blocks: Rayleigh-Benard
+// 256x256x128 FP32 439 -> 412 (94.6 % of a copy's rate), 129x97x75 FP64 112 -> 103, 200x150x90
+// F16 115 -> 102, three sets 110x96x100 FP32 109 -> 96; Kolmogorov 250^3 FP32 440 -> 386.
 #pragma once
 #include <cuda_fp16.h>
 #include <cstdint>
@@ -11,6 +18,11 @@
 namespace ch4 {
 
 constexpr int Q = 19;
+constexpr int POP_BLOCK = 32;
+// values of a population buffer of N cells and `sets` sets (the last block filled up)
+inline size_t pop_values(long long N, int sets) {
+  return (size_t)((N + POP_BLOCK - 1) / POP_BLOCK) * POP_BLOCK * Q * sets;
+}
 constexpr int NK = 6;  // HIT forcing modes, src/initial_conditions.c:841-849
 constexpr int FM_SUMS = 9;     // sums of the global force corrections: F, F*u, u per component
 constexpr int FM_BLOCK = 256;  // threads per block of that reduction
@@ -129,13 +141,11 @@ struct StepParams {
   int Lhit;     // NX + NY + global NZ: length of one HIT table row
   uint32_t feat;
   uint32_t walls;  // W_* bits
-  // populations (storage type erased; cast in the kernel)
+  // populations (storage type erased; cast in the kernel): the first block's values of each
+  // set, and the values of one block (Q * POP_BLOCK times the number of sets)
   const void* fin[3];
   void* fout[3];
-  // plane q of each set (fin[s] + q*N elements), filled by the host with fin/fout: an
-  // access is then one wide multiply-add of the cell index onto a parameter
-  const void* fin_q[3][Q];
-  void* fout_q[3][Q];
+  uint32_t bstride;
   // previous-step temperature / scalar (t^{n-1}), read and overwritten in place
   A* tprev;
   A* sprev;
@@ -192,6 +202,27 @@ struct StepParams {
 };
 
 #ifdef __CUDACC__
+// the value of direction 0 of cell idx in a set's population buffer (direction q: + POP_BLOCK q)
+template <typename S>
+__device__ __forceinline__ const S* pop_at(const void* set, uint32_t bstride, long long idx) {
+  const unsigned int i = (unsigned int)idx;  // cells < 2^31
+  return static_cast<const S*>(set) + (unsigned long long)(i / POP_BLOCK) * bstride + i % POP_BLOCK;
+}
+template <typename S>
+__device__ __forceinline__ S* pop_at(void* set, uint32_t bstride, long long idx) {
+  return const_cast<S*>(pop_at<S>(const_cast<const void*>(set), bstride, idx));
+}
+
+// Programmatic dependent launch: every kernel of the step begins here.  Launched with the
+// attribute (launch_chained) it may be resident before the kernel ahead of it in the stream has
+// ended; it waits for that kernel's end and its writes, then lets the next one come.  What one
+// kernel of the chain writes the next one reads with plain loads: the read-only path promises
+// nothing for data written after a kernel's launch.
+__device__ __forceinline__ void grid_chain() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ---- storage codecs ------------------------------------------------------
 template <typename S, typename A>
 struct Codec;
@@ -199,25 +230,25 @@ struct Codec;
 template <>
 struct Codec<double, double> {
   static constexpr bool deviation = false;
-  __device__ __forceinline__ static double load(const double* p, long long i, double, double) { return __ldg(p + i); }
+  __device__ __forceinline__ static double load(const double* p, long long i, double, double) { return p[i]; }
   __device__ __forceinline__ static void store(double* p, long long i, double v, double, double) { p[i] = v; }
 };
 template <>
 struct Codec<float, float> {
   static constexpr bool deviation = false;
-  __device__ __forceinline__ static float load_raw(const float* p, long long i) { return __ldg(p + i); }
+  __device__ __forceinline__ static float load_raw(const float* p, long long i) { return p[i]; }
   __device__ __forceinline__ static void store_raw(float* p, long long i, float v) { p[i] = v; }
-  __device__ __forceinline__ static float load(const float* p, long long i, float, float) { return __ldg(p + i); }
+  __device__ __forceinline__ static float load(const float* p, long long i, float, float) { return p[i]; }
   __device__ __forceinline__ static void store(float* p, long long i, float v, float, float) { p[i] = v; }
 };
 // IEEE half holding the deviation f_q - w_q * shift
 template <>
 struct Codec<__half, float> {
   static constexpr bool deviation = true;
-  __device__ __forceinline__ static float load_raw(const __half* p, long long i) { return __half2float(__ldg(p + i)); }
+  __device__ __forceinline__ static float load_raw(const __half* p, long long i) { return __half2float(p[i]); }
   __device__ __forceinline__ static void store_raw(__half* p, long long i, float v) { p[i] = __float2half_rn(v); }
   __device__ __forceinline__ static float load(const __half* p, long long i, float w, float shift) {
-    return __half2float(__ldg(p + i)) + w * shift;
+    return __half2float(p[i]) + w * shift;
   }
   __device__ __forceinline__ static void store(__half* p, long long i, float v, float w, float shift) {
     p[i] = __float2half_rn(v - w * shift);

@@ -59,7 +59,18 @@ cudaError_t launch_soa_to_aos(const StepParams<double>& P, LaunchShape s, int se
                               int nz, cudaStream_t st);
 cudaError_t launch_soa_to_aos(const StepParams<float>& P, LaunchShape s, int set, const void* soa, float* aos, int z0,
                               int nz, cudaStream_t st);
-// copies of up to 30 device regions (z-slab face exchange), in 4-byte words when every
+// the populations that cross the z faces of a slab, packed into or unpacked from the face
+// buffers (halo_faces_kernel); `bytes`: of a stored value (2, 4 or 8)
+struct HaloFacesArgs {
+  int NX, NY, NZ, sets;
+  uint32_t own;
+  void* pops;
+  void* down;
+  void* up;
+  bool pack;
+};
+cudaError_t launch_halo_faces(const HaloFacesArgs& a, size_t bytes, cudaStream_t st);
+// copies of up to 30 device regions (the u faces of a z-slab), in 4-byte words when every
 // region's size and addresses allow it, else in 2-byte words
 struct HaloCopy {
   const void* src[30];

@@ -179,12 +179,12 @@ __device__ __forceinline__ int wrap(int v, int n) { return v < 0 ? v + n : (v >=
 // f, rho, ux..u2: the cell's populations and the collision's rho, u^n, |u|^2.
 // the four values of cell c of a (u_x, u_y, u_z, t) array
 __device__ __forceinline__ void ld4(const float* p, long long c, float* v) {
-  const float4 q = __ldg(reinterpret_cast<const float4*>(p) + c);
+  const float4 q = reinterpret_cast<const float4*>(p)[c];
   v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
 }
 __device__ __forceinline__ void ld4(const double* p, long long c, double* v) {
-  const double2 a = __ldg(reinterpret_cast<const double2*>(p) + 2 * c);
-  const double2 b = __ldg(reinterpret_cast<const double2*>(p) + 2 * c + 1);
+  const double2 a = reinterpret_cast<const double2*>(p)[2 * c];
+  const double2 b = reinterpret_cast<const double2*>(p)[2 * c + 1];
   v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
 }
 
@@ -439,6 +439,7 @@ __device__ __forceinline__ void hydro_cell(const StepParams<A>& P, int x, int y,
 template <typename S, typename A, bool THERM, bool SCAL>
 __global__ void hydro_kernel(const StepParams<A> P, const A* hit, const A* dep, const A* fm, double* dens, double* u,
                              double* t, double* s, double* force, A* u_arith, A* ut4, int ut4_t) {
+  grid_chain();
   // one thread per cell whatever NX is, as the step kernel
   const unsigned int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= P.zcells) return;
@@ -489,6 +490,7 @@ __global__ void hydro_kernel(const StepParams<A> P, const A* hit, const A* dep, 
 // update order has it.
 template <typename A>
 __global__ void sism_filter_kernel(const StepParams<A> P) {
+  grid_chain();
   const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (idx >= P.N) return;
   A u[4], m[4];
@@ -576,25 +578,49 @@ __global__ void fields_chunk_kernel(const StepParams<A> P, const A* hit, const A
 // round-to-nearest conversion the storage codec would apply to an FP64 value, so the
 // stored populations are those of an FP64 chunk, with half the bytes on the bus).
 template <typename S, typename A>
-__global__ void aos_to_soa_kernel(const A* aos, S* soa, int NX, int NY, int z0, int nz, long long N, StepParams<A> P,
-                                  int set) {
+__global__ void aos_to_soa_kernel(const A* aos, S* soa, int NX, int NY, int z0, int nz, StepParams<A> P, int set) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long cells = (long long)NX * NY * nz;
   if (t >= cells * Q) return;
   const int q = (int)(t % Q);
   const long long c = t / Q;
-  Codec<S, A>::store(soa, (long long)q * N + (long long)z0 * NX * NY + c, aos[t], P.w[q], P.shift[set]);
+  Codec<S, A>::store(pop_at<S>(soa, P.bstride, (long long)z0 * NX * NY + c), q * POP_BLOCK, aos[t], P.w[q],
+                     P.shift[set]);
 }
 
 template <typename S, typename A>
-__global__ void soa_to_aos_kernel(const S* soa, A* aos, int NX, int NY, int z0, int nz, long long N, StepParams<A> P,
-                                  int set) {
+__global__ void soa_to_aos_kernel(const S* soa, A* aos, int NX, int NY, int z0, int nz, StepParams<A> P, int set) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long cells = (long long)NX * NY * nz;
   if (t >= cells * Q) return;
   const int q = (int)(t % Q);
   const long long c = t / Q;
-  aos[t] = Codec<S, A>::load(soa, (long long)q * N + (long long)z0 * NX * NY + c, P.w[q], P.shift[set]);
+  aos[t] = Codec<S, A>::load(pop_at<S>(soa, P.bstride, (long long)z0 * NX * NY + c), q * POP_BLOCK, P.w[q],
+                             P.shift[set]);
+}
+
+// The populations that cross the z faces of a slab, between the buffer `pops` (its sets one
+// after the other in a block) and the face buffers: direction k of the five with c_z = -1 (top
+// plane, buffer `down`) or +1 (bottom plane, buffer `up`), planes of NX * NY values by set and
+// direction.  Rows whose values the cell's own wall rule writes stay out (own: bit set for a
+// wall above, bit 3 + set for one below).  PACK: populations -> buffers.
+struct HaloFaces {
+  int NX, NY, NZ, sets;
+  uint32_t bstride, own;
+};
+template <typename S, bool PACK>
+__global__ void halo_faces_kernel(S* pops, const HaloFaces H, S* down, S* up) {
+  const long long plane = (long long)H.NX * H.NY, t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t >= plane) return;
+  const int s = blockIdx.y / 10, d = blockIdx.y % 10, y = (int)(t / H.NX);
+  int q = 0;  // the (d mod 5)-th direction with c_z = -1 (d < 5) or +1
+  for (int k = d % 5; q < Q; q++)
+    if (cz(q) == (d < 5 ? -1 : 1) && k-- == 0) break;
+  if ((cy(q) < 0 && y == H.NY - 1 && ((H.own >> s) & 1)) || (cy(q) > 0 && y == 0 && ((H.own >> (3 + s)) & 1))) return;
+  S* cell = pop_at<S>(pops, H.bstride, (d < 5 ? (H.NZ - 1) * plane : 0) + t) + (s * Q + q) * POP_BLOCK;
+  S* face = (d < 5 ? down : up) + ((long long)s * 5 + d % 5) * plane + t;
+  if constexpr (PACK) *face = *cell;
+  else *cell = *face;
 }
 
 #include "force_moments.cuh"

@@ -9,40 +9,25 @@
 //
 // EXACT (the FP64 instantiation) keeps every operation of the reference in its
 // order, so the result is bit-identical.  The FP32 instantiation evaluates the
-// same quantities with fewer instructions (reciprocal density, the equilibrium
-// polynomial in Horner form, the Guo term as (c.F - u.F)/cs^2 + (c.u)(c.F)/cs^4);
-// its error against FP64 is reported, not zero.
+// same quantities as the even and odd parts of pairs of directions; its error
+// against FP64 is reported, not zero.
 
-// Address of plane q of a set.  The half-precision store takes the precomputed plane
-// pointers (fewer integer instructions for the issue-bound form, measured +6 %); the
-// FP32 and FP64 stores compute base + q*N (measured equal for FP32, 11 % faster for FP64).
-template <typename S>
-constexpr bool kPlanePointers = sizeof(S) == 2;
-
-template <typename S, typename A, int set>
-__device__ __forceinline__ const S* plane_in(const StepParams<A>& P, int q) {
-  if constexpr (kPlanePointers<S>) return static_cast<const S*>(P.fin_q[set][q]);
-  return static_cast<const S*>(P.fin[set]) + (long long)q * P.N;
+template <typename S, typename A>
+__device__ __forceinline__ void load_full(const StepParams<A>& P, int set, const S* p, A* f) {
+#pragma unroll
+  for (int q = 0; q < Q; q++) f[q] = Codec<S, A>::load(p, q * POP_BLOCK, P.w[q], P.shift[set]);
 }
-
-template <typename S, typename A, int set>
-__device__ __forceinline__ S* plane_out(const StepParams<A>& P, int q) {
-  if constexpr (kPlanePointers<S>) return static_cast<S*>(P.fout_q[set][q]);
-  return static_cast<S*>(P.fout[set]) + (long long)q * P.N;
-}
-
 template <typename S, typename A, int set>
 __device__ __forceinline__ void load_set(const StepParams<A>& P, long long idx, A* f) {
-#pragma unroll
-  for (int q = 0; q < Q; q++) f[q] = Codec<S, A>::load(plane_in<S, A, set>(P, q), idx, P.w[q], P.shift[set]);
+  load_full(P, set, pop_at<S>(P.fin[set], P.bstride, idx), f);
 }
 
 // The stored values of a cell as they are: f itself, or for the half-precision store the
 // deviation f - w * shift.
-template <typename S, typename A, int set>
-__device__ __forceinline__ void load_raw(const StepParams<A>& P, int idx, A* f) {
+template <typename S, typename A>
+__device__ __forceinline__ void load_raw(const S* p, A* f) {
 #pragma unroll
-  for (int q = 0; q < Q; q++) f[q] = Codec<S, A>::load_raw(plane_in<S, A, set>(P, q), idx);
+  for (int q = 0; q < Q; q++) f[q] = Codec<S, A>::load_raw(p, q * POP_BLOCK);
 }
 
 // the first direction q of pair k = 0 .. 8 of opposite directions (q, qinv(q))
@@ -109,77 +94,97 @@ __device__ __forceinline__ A wall_fac(const StepParams<A>& P, int a, bool plus, 
   return A(2) * (((plus ? P.T_top : P.T_bot) - P.T_ref) - tt);
 }
 
+// direction q of the cell at p
 template <typename S, typename A, bool RAW>
-__device__ __forceinline__ void put(S* plane, int i, A v, A w, A shift) {
-  if constexpr (RAW) Codec<S, A>::store_raw(plane, i, v);
-  else Codec<S, A>::store(plane, i, v, w, shift);
+__device__ __forceinline__ void put(S* p, int q, A v, A w, A shift) {
+  if constexpr (RAW) Codec<S, A>::store_raw(p, q * POP_BLOCK, v);
+  else Codec<S, A>::store(p, q * POP_BLOCK, v, w, shift);
 }
 
-// push one set; wallmode: 0 no walls, 1 fluid walls, 2 value walls (temperature or scalar).
-// WALLS = false is the form for cells that touch no wall: every value streams to x + c_q.
+// The push of a cell that meets no wall: every value streams to x + c_q, the sets of a
+// direction to one address.
+template <typename S, typename A, bool THERM, bool SCAL, bool RAW, int q>
+__device__ __forceinline__ void push_bulk_one(const StepParams<A>& P, int idx, const Nbr& nb, const A* f, const A* g,
+                                              const A* h) {
+  constexpr int sets = 1 + (THERM ? 1 : 0) + (SCAL ? 1 : 0);
+  S* p = pop_at<S>(P.fout[0], sets * Q * POP_BLOCK, idx + nbr_delta<q, true>(nb));
+  put<S, A, RAW>(p, q, f[q], P.w[q], RAW ? A(0) : A(P.shift[0]));
+  if constexpr (THERM) put<S, A, RAW>(p, Q + q, g[q], P.w[q], RAW ? A(0) : A(P.shift[1]));
+  if constexpr (SCAL) put<S, A, RAW>(p, (sets - 1) * Q + q, h[q], P.w[q], RAW ? A(0) : A(P.shift[2]));
+}
+template <typename S, typename A, bool THERM, bool SCAL, bool RAW>
+__device__ __forceinline__ void push_bulk(const StepParams<A>& P, int idx, const Nbr& nb, const A* f, const A* g,
+                                          const A* h) {
+#define CH4_PUSH(Q_) push_bulk_one<S, A, THERM, SCAL, RAW, Q_>(P, idx, nb, f, g, h);
+  CH4_PUSH(0) CH4_PUSH(1) CH4_PUSH(2) CH4_PUSH(3) CH4_PUSH(4) CH4_PUSH(5) CH4_PUSH(6) CH4_PUSH(7) CH4_PUSH(8)
+  CH4_PUSH(9) CH4_PUSH(10) CH4_PUSH(11) CH4_PUSH(12) CH4_PUSH(13) CH4_PUSH(14) CH4_PUSH(15) CH4_PUSH(16)
+  CH4_PUSH(17) CH4_PUSH(18)
+#undef CH4_PUSH
+}
+
+// The push of one set of a cell on a wall; wallmode: 0 no walls of this set, 1 fluid walls,
+// 2 value walls (temperature or scalar).
 // RAW: `post` holds values as they are stored (a wall rule moves a value between directions
 // of the same weight, so the deviation form passes through it unchanged).
-template <typename S, typename A, int set, int q, bool WALLS, bool RAW>
+template <typename S, typename A, int set, int q, bool RAW>
 __device__ __forceinline__ void push_one(const StepParams<A>& P, int idx, const Nbr& nb, const A* post, int wallmode,
                                          const Walls& W, A tt, A ss) {
   const A sh = RAW ? A(0) : A(P.shift[set]);
-  if constexpr (WALLS) {
-    // the wall bit of each axis this direction leaves through (compile-time masks: q is fixed)
-    constexpr uint32_t mx = cx(q) > 0 ? 1u : cx(q) < 0 ? 8u : 0u;
-    constexpr uint32_t my = cy(q) > 0 ? 2u : cy(q) < 0 ? 16u : 0u;
-    constexpr uint32_t mz = cz(q) > 0 ? 4u : cz(q) < 0 ? 32u : 0u;
-    const bool hx = (W.hit & mx) != 0, hy = (W.hit & my) != 0, hz = (W.hit & mz) != 0;
-    if (wallmode != 0 && (hx || hy || hz)) {
-      if (wallmode == 1) {
-        // a slip wall stands alone on its axis (the other axes are periodic), so a direction
-        // that meets it meets no other wall
-        if (int(hx) + int(hy) + int(hz) == 1) {
-          const bool sx = (W.slip & mx) != 0, sy = (W.slip & my) != 0, sz = (W.slip & mz) != 0;
-          // specular reflection: the hit axis keeps the cell's coordinate, the others stream
-          // (src/boundary_conditions.c:606-610 (x), 751-753 (y), 895-899 (z))
-          if (hx && sx) {
-            constexpr int r = qmirror(q, 0);
-            const int d = (cy(q) < 0 ? nb.ym : cy(q) > 0 ? nb.yp : 0) + (cz(q) < 0 ? nb.zm : cz(q) > 0 ? nb.zp : 0);
-            put<S, A, RAW>(plane_out<S, A, set>(P, r), idx + d, post[q], P.w[r], sh);
-            return;
-          }
-          if (hy && sy) {
-            constexpr int r = qmirror(q, 1);
-            put<S, A, RAW>(plane_out<S, A, set>(P, r), idx + nbr_delta<q, false>(nb), post[q], P.w[r], sh);
-            return;
-          }
-          if (hz && sz) {
-            constexpr int r = qmirror(q, 2);
-            const int d = (cx(q) < 0 ? nb.xm : cx(q) > 0 ? nb.xp : 0) + (cy(q) < 0 ? nb.ym : cy(q) > 0 ? nb.yp : 0);
-            put<S, A, RAW>(plane_out<S, A, set>(P, r), idx + d, post[q], P.w[r], sh);
-            return;
-          }
+  // the wall bit of each axis this direction leaves through (compile-time masks: q is fixed)
+  constexpr uint32_t mx = cx(q) > 0 ? 1u : cx(q) < 0 ? 8u : 0u;
+  constexpr uint32_t my = cy(q) > 0 ? 2u : cy(q) < 0 ? 16u : 0u;
+  constexpr uint32_t mz = cz(q) > 0 ? 4u : cz(q) < 0 ? 32u : 0u;
+  const bool hx = (W.hit & mx) != 0, hy = (W.hit & my) != 0, hz = (W.hit & mz) != 0;
+  if (wallmode != 0 && (hx || hy || hz)) {
+    if (wallmode == 1) {
+      // a slip wall stands alone on its axis (the other axes are periodic), so a direction
+      // that meets it meets no other wall
+      if (int(hx) + int(hy) + int(hz) == 1) {
+        const bool sx = (W.slip & mx) != 0, sy = (W.slip & my) != 0, sz = (W.slip & mz) != 0;
+        // specular reflection: the hit axis keeps the cell's coordinate, the others stream
+        // (src/boundary_conditions.c:606-610 (x), 751-753 (y), 895-899 (z))
+        if (hx && sx) {
+          constexpr int r = qmirror(q, 0);
+          const int d = (cy(q) < 0 ? nb.ym : cy(q) > 0 ? nb.yp : 0) + (cz(q) < 0 ? nb.zm : cz(q) > 0 ? nb.zp : 0);
+          put<S, A, RAW>(pop_at<S>(P.fout[set], P.bstride, idx + d), r, post[q], P.w[r], sh);
+          return;
         }
-        // halfway bounce-back, src/boundary_conditions.c:623,775,917
-        constexpr int r = qinv(q);
-        put<S, A, RAW>(plane_out<S, A, set>(P, r), idx, post[q], P.w[r], sh);
-      } else {
-        // fixed value / flux walls: the reference's loops run y, then x, then z, each writing
-        // the slot the cell pulls as inv[q]; the last wall the direction crosses decides
-        // (src/boundary_conditions.c:1019-1027, 1118-1151, 1186-1224).  Temperature walls on
-        // x store rhs(x).p[q] + w[inv q] fac, every other value wall rhs(x).p[inv q] + ...
-        constexpr int r = qinv(q);
-        const int a = hz ? 2 : hx ? 0 : 1;
-        const bool plus = a == 2 ? cz(q) > 0 : a == 0 ? cx(q) > 0 : cy(q) > 0;
-        const A fac = wall_fac<set>(P, a, plus, tt, ss);
-        const A base = (set == 1 && a == 0) ? post[q] : post[r];
-        put<S, A, RAW>(plane_out<S, A, set>(P, r), idx, base + P.w[r] * fac, P.w[r], sh);
+        if (hy && sy) {
+          constexpr int r = qmirror(q, 1);
+          put<S, A, RAW>(pop_at<S>(P.fout[set], P.bstride, idx + nbr_delta<q, false>(nb)), r, post[q], P.w[r], sh);
+          return;
+        }
+        if (hz && sz) {
+          constexpr int r = qmirror(q, 2);
+          const int d = (cx(q) < 0 ? nb.xm : cx(q) > 0 ? nb.xp : 0) + (cy(q) < 0 ? nb.ym : cy(q) > 0 ? nb.yp : 0);
+          put<S, A, RAW>(pop_at<S>(P.fout[set], P.bstride, idx + d), r, post[q], P.w[r], sh);
+          return;
+        }
       }
-      return;
+      // halfway bounce-back, src/boundary_conditions.c:623,775,917
+      constexpr int r = qinv(q);
+      put<S, A, RAW>(pop_at<S>(P.fout[set], P.bstride, idx), r, post[q], P.w[r], sh);
+    } else {
+      // fixed value / flux walls: the reference's loops run y, then x, then z, each writing
+      // the slot the cell pulls as inv[q]; the last wall the direction crosses decides
+      // (src/boundary_conditions.c:1019-1027, 1118-1151, 1186-1224).  Temperature walls on
+      // x store rhs(x).p[q] + w[inv q] fac, every other value wall rhs(x).p[inv q] + ...
+      constexpr int r = qinv(q);
+      const int a = hz ? 2 : hx ? 0 : 1;
+      const bool plus = a == 2 ? cz(q) > 0 : a == 0 ? cx(q) > 0 : cy(q) > 0;
+      const A fac = wall_fac<set>(P, a, plus, tt, ss);
+      const A base = (set == 1 && a == 0) ? post[q] : post[r];
+      put<S, A, RAW>(pop_at<S>(P.fout[set], P.bstride, idx), r, base + P.w[r] * fac, P.w[r], sh);
     }
+    return;
   }
-  put<S, A, RAW>(plane_out<S, A, set>(P, q), idx + nbr_delta<q, true>(nb), post[q], P.w[q], sh);
+  put<S, A, RAW>(pop_at<S>(P.fout[set], P.bstride, idx + nbr_delta<q, true>(nb)), q, post[q], P.w[q], sh);
 }
 
-template <typename S, typename A, int set, bool WALLS, bool RAW>
+template <typename S, typename A, int set, bool RAW>
 __device__ __forceinline__ void push_set(const StepParams<A>& P, int idx, const Nbr& nb, const A* post, int wallmode,
                                          const Walls& W, A tt, A ss) {
-#define CH4_PUSH(Q_) push_one<S, A, set, Q_, WALLS, RAW>(P, idx, nb, post, wallmode, W, tt, ss);
+#define CH4_PUSH(Q_) push_one<S, A, set, Q_, RAW>(P, idx, nb, post, wallmode, W, tt, ss);
   CH4_PUSH(0) CH4_PUSH(1) CH4_PUSH(2) CH4_PUSH(3) CH4_PUSH(4) CH4_PUSH(5) CH4_PUSH(6) CH4_PUSH(7) CH4_PUSH(8)
   CH4_PUSH(9) CH4_PUSH(10) CH4_PUSH(11) CH4_PUSH(12) CH4_PUSH(13) CH4_PUSH(14) CH4_PUSH(15) CH4_PUSH(16)
   CH4_PUSH(17) CH4_PUSH(18)
@@ -193,7 +198,7 @@ __device__ __forceinline__ void push_set(const StepParams<A>& P, int idx, const 
 template <typename S, typename A, int set, bool RAW>
 __device__ __noinline__ void push_walled(const StepParams<A>& P, int idx, Nbr nb, const A* post, int wallmode,
                                          Walls W, A tt, A ss) {
-  push_set<S, A, set, true, RAW>(P, idx, nb, post, wallmode, W, tt, ss);
+  push_set<S, A, set, RAW>(P, idx, nb, post, wallmode, W, tt, ss);
 }
 
 // Per-cell quantities shared by the collision of every direction.
@@ -545,10 +550,12 @@ __device__ __forceinline__ void lb_cell(const StepParams<A>& P, int x, int y, in
     tl = les_tau<EXACT>(P, x, y, z, idx, f, rho, ul[0], ul[1], ul[2], u2);
     P.tau_les[idx] = tl;
   }
+  constexpr int sets = 1 + (THERM ? 1 : 0) + (SCAL ? 1 : 0);
+  const S* p = pop_at<S>(P.fin[0], sets * Q * POP_BLOCK, idx);
   if constexpr (RAW) {
-    load_raw<S, A, 0>(P, idx, f);
-    if constexpr (THERM) load_raw<S, A, 1>(P, idx, g);
-    if constexpr (SCAL) load_raw<S, A, 2>(P, idx, h);
+    load_raw(p, f);
+    if constexpr (THERM) load_raw(p + Q * POP_BLOCK, g);
+    if constexpr (SCAL) load_raw(p + (sets - 1) * Q * POP_BLOCK, h);
     constexpr bool DEV = Codec<S, A>::deviation;
     moments32(f, c.dr, mx, my, mz);
     c.dt = THERM ? sum32(g) : A(0);
@@ -557,9 +564,9 @@ __device__ __forceinline__ void lb_cell(const StepParams<A>& P, int x, int y, in
     c.tt = DEV && THERM ? c.dt + P.shift[1] : c.dt;
     c.ss = DEV && SCAL ? c.ds + P.shift[2] : c.ds;
   } else {
-    load_set<S, A, 0>(P, idx, f);
-    if constexpr (THERM) load_set<S, A, 1>(P, idx, g);
-    if constexpr (SCAL) load_set<S, A, 2>(P, idx, h);
+    load_full(P, 0, p, f);
+    if constexpr (THERM) load_full(P, 1, p + Q * POP_BLOCK, g);
+    if constexpr (SCAL) load_full(P, 2, p + (sets - 1) * Q * POP_BLOCK, h);
     c.rho = c.dr = mom0(f);
     mx = momx(f), my = momy(f), mz = momz(f);
     c.tt = c.dt = THERM ? mom0(g) : A(0);
@@ -623,16 +630,15 @@ __device__ __forceinline__ void lb_cell(const StepParams<A>& P, int x, int y, in
   const uint32_t WL = P.walls;
   const bool toprow = y == P.NY - 1, botrow = y == 0;
   const bool xedge = (WL & (W_FX | W_TX | W_SX)) && (x == 0 || x == P.NX - 1);
+  const bool yedge = (F & (K_FWALL | K_TWALL | K_SWALL)) && (toprow || botrow);
   const bool zedge = (WL & (W_FZ | W_TZ | W_SZ)) && (z == 0 || z == P.NZ - 1);
   Walls W{0u, 0u};
-#ifndef CH4_NO_WALL_SPLIT
-  if (!(toprow || botrow || xedge || zedge)) {  // cells that touch no wall stream every value
-    push_set<S, A, 0, false, RAW>(P, idx, nb, f, 0, W, c.tt, c.ss);
-    if constexpr (THERM) push_set<S, A, 1, false, RAW>(P, idx, nb, g, 0, W, c.tt, c.ss);
-    if constexpr (SCAL) push_set<S, A, 2, false, RAW>(P, idx, nb, h, 0, W, c.tt, c.ss);
+  // cells that touch no wall stream every value (periodic y rows too: Kolmogorov 32^3 FP32, where
+  // the rows' out-of-line push ended the step, 6.2 -> 4.6 us)
+  if (!(xedge || yedge || zedge)) {
+    push_bulk<S, A, THERM, SCAL, RAW>(P, idx, nb, f, g, h);
     return;
   }
-#endif
   // the wall bits of this cell for walls on the axes (x, y, z) of a set
   const uint32_t at = (x == P.NX - 1 ? 1u : 0u) | (toprow ? 2u : 0u) | (z == P.NZ - 1 ? 4u : 0u) |
                       (x == 0 ? 8u : 0u) | (botrow ? 16u : 0u) | (z == 0 ? 32u : 0u);
@@ -666,6 +672,7 @@ __device__ __forceinline__ void lb_cell(const StepParams<A>& P, int x, int y, in
 // coordinates.  Rayleigh-Benard 129x97x75 FP64: 142 -> 112 us a step (with the pairs above).
 template <typename S, typename A, bool THERM, bool SCAL, int V>
 __device__ __forceinline__ void lb_thread(const StepParams<A>& P) {
+  grid_chain();
   const unsigned int i = blockIdx.x * (unsigned)blockDim.x + threadIdx.x;
   if (i >= P.zcells) return;
   const unsigned int k = fast_div(i, P.div_nxy), r = i - k * (unsigned)(P.NX * P.NY);
@@ -678,20 +685,22 @@ __global__ void __launch_bounds__(128) lb_step_kernel(const __grid_constant__ St
   lb_thread<S, A, THERM, SCAL, V>(P);
 }
 
-// FP32 arithmetic, fluid + temperature, Smagorinsky LES: held to 64 registers (eight
-// 128-thread blocks per SM) it runs 8-11 % faster than at the 88 it takes unbounded, a few
-// spilled values included (measured on Rayleigh-Benard LES at 96^3 and 192^3; the
-// single-set LES kernel already fits 64, the 80-register bound measured slower)
-template <typename S, typename A, bool THERM, bool SCAL, int V>
-__global__ void __launch_bounds__(128, 8) lb_step_kernel_les64(const __grid_constant__ StepParams<A> P) {
-  lb_thread<S, A, THERM, SCAL, V>(P);
+// Resident 128-thread blocks per SM that a form is held to, 0 where the compiler's own choice
+// stands (a hint then raises the registers).  The forms run at the HBM roofline or wait for
+// it, and lose with fewer warps; at these bounds none spills more than 8 bytes.  us a step:
+//   FP64, two sets: 4 (128 registers), 13 % over the 3 that a few registers more leave
+//   FP32, fluid only 250^3: 390.3 -> 386.5 at 10 blocks (48 registers); at 8: 409.7
+//   FP32, two sets 256x256x128: 414.1 -> 412.1 at 7 blocks (72); at 5: 429.7; F16 301.6 ->
+//   296.7; with LES 128^3 156.2 -> 151.7; three sets: 5
+template <typename A, bool THERM, bool SCAL, int V>
+constexpr int step_blocks() {
+  constexpr int sets = 1 + (THERM ? 1 : 0) + (SCAL ? 1 : 0);
+  if (V & V_TRT) return 0;
+  if (sizeof(A) == 8) return V == 0 && sets == 2 ? 4 : 0;
+  return sets == 1 ? (V == 0 ? 10 : 0) : sets == 2 ? 7 : 5;
 }
-
-// The FP64 BGK step with two population sets, held to 128 registers (four 128-thread
-// blocks per SM): the allocation at which it runs at the HBM roofline; left to itself the
-// compiler may take a few more and lose a block per SM (-13 % measured).  (A minimum-blocks
-// hint on the other forms raises their registers instead; they keep the plain bound.)
-template <typename S, typename A, bool THERM, bool SCAL>
-__global__ void __launch_bounds__(128, 4) lb_step_kernel_cap128(const __grid_constant__ StepParams<A> P) {
-  lb_thread<S, A, THERM, SCAL, 0>(P);
+template <typename S, typename A, bool THERM, bool SCAL, int V>
+__global__ void __launch_bounds__(128, step_blocks<A, THERM, SCAL, V>()) lb_step_kernel_blocks(
+    const __grid_constant__ StepParams<A> P) {
+  lb_thread<S, A, THERM, SCAL, V>(P);
 }

@@ -221,16 +221,16 @@ __device__ __forceinline__ int pmod(int i, int n) {
 }
 
 // the four values (u_x, u_y, u_z, t) of cell c of ut4: FP32 as one 16-byte load, FP64 as two
-__device__ __forceinline__ void load_cell(const float* __restrict__ ut4, long long c, double* v) {
-  const float4 q = __ldg(reinterpret_cast<const float4*>(ut4) + c);
+__device__ __forceinline__ void load_cell(const float* ut4, long long c, double* v) {
+  const float4 q = reinterpret_cast<const float4*>(ut4)[c];
   v[0] = q.x;
   v[1] = q.y;
   v[2] = q.z;
   v[3] = q.w;
 }
-__device__ __forceinline__ void load_cell(const double* __restrict__ ut4, long long c, double* v) {
-  const double2 a = __ldg(reinterpret_cast<const double2*>(ut4) + 2 * c);
-  const double2 b = __ldg(reinterpret_cast<const double2*>(ut4) + 2 * c + 1);
+__device__ __forceinline__ void load_cell(const double* ut4, long long c, double* v) {
+  const double2 a = reinterpret_cast<const double2*>(ut4)[2 * c];
+  const double2 b = reinterpret_cast<const double2*>(ut4)[2 * c + 1];
   v[0] = a.x;
   v[1] = a.y;
   v[2] = b.x;
@@ -418,7 +418,7 @@ __host__ __device__ constexpr int corners_done(int axis, int l) {
 }
 
 template <int NF, typename C>
-__device__ __forceinline__ void load_line(const C* __restrict__ ut4, const PBlock& o, int axis, int a, int b,
+__device__ __forceinline__ void load_line(const C* ut4, const PBlock& o, int axis, int a, int b,
                                           C (*L)[NF]) {
 #pragma unroll
   for (int q = 0; q < 4; q++) {
@@ -830,6 +830,7 @@ __device__ __forceinline__ void deposit_rows_emit(const PartParams<A>& P, int ip
 // FP32: four blocks of 128 per SM (<= 128 registers); FP64 keeps twice the registers
 template <typename A, bool ORIENT, bool HALO, int NF>
 __global__ void __launch_bounds__(128, sizeof(A) == 8 ? 2 : 4) particle_substep_kernel(const PartParams<A> P) {
+  grid_chain();
   const int ip = blockIdx.x * blockDim.x + threadIdx.x;
   if (ip >= P.np) return;
   double* pf = P.pf;
@@ -1182,7 +1183,8 @@ __global__ void particle_key_kernel(const PartParams<A> P) {
 // particles (pf_alt holds the others since the upload).  HBM-bound: 16 bytes a plane and
 // particle; of the 75 planes a two-way run without orientation or temperature moves 40.
 template <typename A>
-__global__ void particle_permute_kernel(const PartParams<A> P, const PartPlanes L, const int* __restrict__ src) {
+__global__ void particle_permute_kernel(const PartParams<A> P, const PartPlanes L, const int* src) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= P.np) return;
   const long long np = P.np;

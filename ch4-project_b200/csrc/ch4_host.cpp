@@ -1783,10 +1783,14 @@ struct Engine : EngineBase {
     ch4_status st;
     const bool hit = (c.flags & CH4_F_FORCING_HIT) != 0;
     const size_t slot = (size_t)NK * L();
-    int done = 0;
+    int done = 0, span = 8;
     while (done < n) {
+      // The host forms the phase tables of a chunk of steps (18 sines per lattice row, plane and
+      // column a step) before it launches them: the first chunks are short, so that the device
+      // starts at once and the later ones are formed while it works.
       // (orientation noise draws from the stream between two phase walks: one step at a time)
-      const int m = (noise() || rj_random()) ? 1 : std::min(CHUNK, n - done);
+      const int m = (noise() || rj_random()) ? 1 : std::min(hit ? std::min(span, CHUNK) : CHUNK, n - done);
+      if (span < CHUNK) span *= 2;
       if (hit) {
         // tables for phi_n (slot 0 = latest) and the m next phase sets
         if ((st = H->cuda(cudaEventSynchronize(hit_ev), "hit event"))) return st;

@@ -217,7 +217,9 @@ __device__ __forceinline__ S* pop_at(void* set, uint32_t bstride, long long idx)
 // attribute (launch_chained) it may be resident before the kernel ahead of it in the stream has
 // ended; it waits for that kernel's end and its writes, then lets the next one come.  What one
 // kernel of the chain writes the next one reads with plain loads: the read-only path promises
-// nothing for data written after a kernel's launch.
+// nothing for data written after a kernel's launch.  The gap between two dependent kernels was
+// 2 us: us a step, Kolmogorov 32^3 FP32 4.7 -> 3.4, 64^3 FP32 10.3 -> 6.9, 64^3 FP64 14.6 ->
+// 12.8, Rayleigh-Benard 32^3 FP32 10.3 -> 7.8, LES with tracers 96^3 62 -> 55.
 __device__ __forceinline__ void grid_chain() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

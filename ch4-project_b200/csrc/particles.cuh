@@ -221,16 +221,16 @@ __device__ __forceinline__ int pmod(int i, int n) {
 }
 
 // the four values (u_x, u_y, u_z, t) of cell c of ut4: FP32 as one 16-byte load, FP64 as two
-__device__ __forceinline__ void load_cell(const float* ut4, long long c, double* v) {
-  const float4 q = reinterpret_cast<const float4*>(ut4)[c];
+__device__ __forceinline__ void load_cell(const float* __restrict__ ut4, long long c, double* v) {
+  const float4 q = __ldg(reinterpret_cast<const float4*>(ut4) + c);
   v[0] = q.x;
   v[1] = q.y;
   v[2] = q.z;
   v[3] = q.w;
 }
-__device__ __forceinline__ void load_cell(const double* ut4, long long c, double* v) {
-  const double2 a = reinterpret_cast<const double2*>(ut4)[2 * c];
-  const double2 b = reinterpret_cast<const double2*>(ut4)[2 * c + 1];
+__device__ __forceinline__ void load_cell(const double* __restrict__ ut4, long long c, double* v) {
+  const double2 a = __ldg(reinterpret_cast<const double2*>(ut4) + 2 * c);
+  const double2 b = __ldg(reinterpret_cast<const double2*>(ut4) + 2 * c + 1);
   v[0] = a.x;
   v[1] = a.y;
   v[2] = b.x;
@@ -418,7 +418,7 @@ __host__ __device__ constexpr int corners_done(int axis, int l) {
 }
 
 template <int NF, typename C>
-__device__ __forceinline__ void load_line(const C* ut4, const PBlock& o, int axis, int a, int b,
+__device__ __forceinline__ void load_line(const C* __restrict__ ut4, const PBlock& o, int axis, int a, int b,
                                           C (*L)[NF]) {
 #pragma unroll
   for (int q = 0; q < 4; q++) {
@@ -874,6 +874,16 @@ __global__ void __launch_bounds__(128, sizeof(A) == 8 ? 2 : 4) particle_substep_
     }
   }
   const double ux = v[0], uy = v[1], uz = v[2];
+  // everything the push reads of the state, before the first store: the loads go out together
+  // (after a store to the same arrays each would wait for its turn; 250,000 particles in 160^3
+  // FP32: 423 -> 405 us a step)
+  const double vx0 = F(vx), vy0 = F(vy), vz0 = F(vz);
+  const double tau = F(tau_drag), beta = F(beta_coeff);
+  const double vxp = F(vx_old), vyp = F(vy_old), vzp = F(vz_old);
+  const double uxp = F(ux_old), uyp = F(uy_old), uzp = F(uz_old);
+  const double axp = F(ax_old), ayp = F(ay_old), azp = F(az_old);
+  [[maybe_unused]] double t_old = 0.0;
+  if constexpr (NF == 4) t_old = F(t_old);
   F(ux) = ux;
   F(uy) = uy;
   F(uz) = uz;
@@ -899,8 +909,6 @@ __global__ void __launch_bounds__(128, sizeof(A) == 8 ? 2 : 4) particle_substep_
     gr[2][2] = F(dz_uz);
   }
   // ---- move_particles (src/lagrange.c:2934-3470)
-  const double vx0 = F(vx), vy0 = F(vy), vz0 = F(vz);
-  const double tau = F(tau_drag), beta = F(beta_coeff);
   const double dtl = P.dtl;
   const bool first = P.first != 0;
   if constexpr (NF == 4) {
@@ -914,7 +922,7 @@ __global__ void __launch_bounds__(128, sizeof(A) == 8 ? 2 : 4) particle_substep_
     if (first) {
       F(t_old) = tv;
     } else {
-      const double dt_t = (tv - F(t_old)) / dtl;
+      const double dt_t = (tv - t_old) / dtl;
       F(dt_t) = dt_t;
       F(t_old) = tv;
       if (P.gradient) F(Dt_t) = dt_t + (ux - vx0) * gr[3][0] + (uy - vy0) * gr[3][1] + (uz - vz0) * gr[3][2];
@@ -934,7 +942,7 @@ __global__ void __launch_bounds__(128, sizeof(A) == 8 ? 2 : 4) particle_substep_
     vz = uz;
     if constexpr (ORIENT)  // active tracers need LAGRANGE_ORIENTATION
       if (P.swim) swim_velocity(pf, np, ip, P.swim, P.jump_flags, P.log001, dtl, vx, vy, vz);
-    double vxo = F(vx_old), vyo = F(vy_old), vzo = F(vz_old);
+    double vxo = vxp, vyo = vyp, vzo = vzp;
     if (first) {
       vxo = vx;
       vyo = vy;
@@ -986,7 +994,7 @@ __global__ void __launch_bounds__(128, sizeof(A) == 8 ? 2 : 4) particle_substep_
         ay -= (-beta) * gc * P.g[1];
         az -= (-beta) * gc * P.g[2];
       }
-      double uxo = F(ux_old), uyo = F(uy_old), uzo = F(uz_old);
+      double uxo = uxp, uyo = uyp, uzo = uzp;
       if (first) {
         uxo = ux;
         uyo = uy;
@@ -1002,7 +1010,7 @@ __global__ void __launch_bounds__(128, sizeof(A) == 8 ? 2 : 4) particle_substep_
       F(Dt_uy) = Dy;
       F(Dt_uz) = Dz;
     }
-    const double vxo = F(vx_old), vyo = F(vy_old), vzo = F(vz_old);
+    const double vxo = vxp, vyo = vyp, vzo = vzp;
     if (first) {
       xn = x0 + dtl * vx;
       yn = y0 + dtl * vy;
@@ -1023,9 +1031,9 @@ __global__ void __launch_bounds__(128, sizeof(A) == 8 ? 2 : 4) particle_substep_
       vy += dtl * ay;
       vz += dtl * az;
     } else {
-      vx += dtl * 0.5 * (3.0 * ax - F(ax_old));
-      vy += dtl * 0.5 * (3.0 * ay - F(ay_old));
-      vz += dtl * 0.5 * (3.0 * az - F(az_old));
+      vx += dtl * 0.5 * (3.0 * ax - axp);
+      vy += dtl * 0.5 * (3.0 * ay - ayp);
+      vz += dtl * 0.5 * (3.0 * az - azp);
     }
     if (P.addedmass && beta != 0.0) {
       dep_have = true;

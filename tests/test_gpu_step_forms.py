@@ -18,8 +18,8 @@ STEPS = 4
 
 
 @pytest.mark.parametrize("storage", [1, 2], ids=["f32", "f16"])
-@pytest.mark.parametrize("name", ["kolmogorov", "rb", "scalar", "les"])
-@pytest.mark.parametrize("dims", [(33, 5, 4), (129, 4, 3), (31, 7, 6), (3, 43, 1), (128, 3, 3)])
+@pytest.mark.parametrize("name", ["kolmogorov", "rb", "scalar", "les", "les_vd", "les_ts"])
+@pytest.mark.parametrize("dims", [(33, 5, 4), (129, 4, 3), (31, 7, 6), (3, 43, 1), (128, 3, 3), (34, 9, 33)])
 def test_step_forms(name, dims, storage):
     _, cfg, state = make_case(name, seed=3, storage=storage, dims=dims)
     ref = run_restatement(cfg, state, STEPS)

@@ -20,6 +20,7 @@
 constexpr int ROW_SEG = 256;    // cells of a row that one warp owns
 constexpr int ROW_CHUNK = 64;   // merged entries in shared memory at a time (8 lists x 8)
 constexpr int ROW_WARPS = 4;    // warps per block
+constexpr int ROW_COPY = 64;    // records per block of row_lists_kernel, ROW_REC / 2 threads each
 constexpr int ROW_REC = 10;     // doubles of a record: fac*fp (3), dxm dxp dym dyp dzm dzp, {hx, index}
 
 // row segments along x: the last home cell (hx = NX) belongs to the last segment
@@ -100,9 +101,9 @@ static __global__ void row_lists_kernel(const unsigned int* key, const int* slot
                                         int copies, const double2* rec, double2* srec, int* start) {
   grid_chain();
   if ((int)blockIdx.x < copies) {
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const int i = (int)(t / (ROW_REC / 2)), part = (int)(t % (ROW_REC / 2));
-    if (i < n && key[i] < nb) srec[t] = rec[(long long)slot[i] * (ROW_REC / 2) + part];
+    const int i = blockIdx.x * ROW_COPY + threadIdx.x / (ROW_REC / 2), part = threadIdx.x % (ROW_REC / 2);
+    if (i < n && key[i] < nb)
+      srec[(long long)i * (ROW_REC / 2) + part] = rec[(long long)slot[i] * (ROW_REC / 2) + part];
     return;
   }
   const unsigned int b = (blockIdx.x - (unsigned)copies) * blockDim.x + threadIdx.x;
@@ -123,6 +124,41 @@ __host__ __device__ __forceinline__ int row_shared(int NX) {
   return ROW_CHUNK * 6 * 8 + 3 * row_cells(NX) * 8 + ROW_CHUNK * 2 * 4;
 }
 
+// what a record of list l adds to the two cells it has in the row: component c of corner di at
+// o[2 c + di]; *x: the cell of corner 0 (corner 1: the one before)
+__device__ __forceinline__ void row_entry(const double2* r, int l, int x0, double* o, int* x) {
+  const double wy = (l & 1) ? r[3].x : r[2].y;         // dyp : dym
+  const double wz = ((l >> 1) & 1) ? r[4].x : r[3].y;  // dzp : dzm
+  const double v0 = r[1].y * wy * wz, v1 = r[2].x * wy * wz;
+  o[0] = r[0].x * v0;
+  o[1] = r[0].x * v1;
+  o[2] = r[0].y * v0;
+  o[3] = r[0].y * v1;
+  o[4] = r[1].x * v0;
+  o[5] = r[1].x * v1;
+  *x = __double2loint(r[4].y) - x0;
+}
+
+// the merged entries in particle order: lane 2 c + di adds component c to the corner di
+__device__ __forceinline__ void row_accumulate(int merged, int lane, int n, int cells, const double* con,
+                                               const int* s_x, double* acc) {
+  for (int e0 = 0; e0 < merged; e0 += 4) {
+    int cell[4];
+    double v[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int e = min(e0 + q, merged - 1);
+      cell[q] = e0 + q < merged && lane < 6 ? s_x[e] - (lane & 1) : -1;
+      v[q] = con[6 * e + (lane < 6 ? lane : 0)];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      if (cell[q] >= 0 && cell[q] < n) acc[(lane >> 1) * cells + cell[q]] += v[q];
+      __syncwarp();
+    }
+  }
+}
+
 template <typename A>
 __global__ void __launch_bounds__(32 * ROW_WARPS) deposit_rows_kernel(const PartParams<A> P) {
   grid_chain();
@@ -132,10 +168,10 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) deposit_rows_kernel(const Part
   double* const acc = con + ROW_CHUNK * 6;
   int* const s_pid = reinterpret_cast<int*>(acc + 3 * cells);
   int* const s_x = s_pid + ROW_CHUNK;
-  const int ns = row_segs(P.NX);
-  const long long w = (long long)blockIdx.x * ROW_WARPS + warp;
-  if (w >= (long long)ns * P.NY * P.NZ) return;  // whole warps: no block barrier below
-  const int seg = (int)(w % ns), j = (int)((w / ns) % P.NY), k = (int)(w / ((long long)ns * P.NY));
+  const int ns = row_segs(P.NX), nl = ns == 1 ? 4 : 8;  // lists
+  const unsigned int w = blockIdx.x * ROW_WARPS + warp;  // of plane k's ns * NY
+  const int j = (int)(ns == 1 ? w : w / (unsigned)ns), seg = (int)w - j * ns, k = blockIdx.y;
+  if (j >= P.NY) return;  // whole warps: no block barrier below
   const int x0 = seg * ROW_SEG, n = min(ROW_SEG, P.NX - x0);
   A* out = P.dep + ((long long)k * P.NY + j) * P.NX + x0;
   // lane l < 4: the home row (y + (l & 1), z + (l >> 1)) of this segment; 4 <= l < 8: the same
@@ -150,6 +186,33 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) deposit_rows_kernel(const Part
   constexpr unsigned ALL = 0xffffffffu;
   if (__any_sync(ALL, beg < end)) {
     for (int c = lane; c < n; c += 32) acc[c] = acc[cells + c] = acc[2 * cells + c] = 0.0;
+    const int all = __reduce_add_sync(ALL, end - beg);
+    if (all <= 32) {
+      // one entry per lane, ranked by comparing it with every other
+      int off = end - beg;
+#pragma unroll
+      for (int d = 1; d < 8; d <<= 1) {
+        const int v = __shfl_up_sync(ALL, off, d);
+        if (lane >= d && lane < 8) off += v;
+      }
+      off -= end - beg;
+      int l = 0;
+      for (int q = 1; q < nl; q++)  // the last list that begins at or before this lane
+        if (__shfl_sync(ALL, off, q) <= lane) l = q;
+      const int pos = __shfl_sync(ALL, beg, l) - __shfl_sync(ALL, off, l) + lane;
+      const bool on = lane < all;
+      const double2* r = reinterpret_cast<const double2*>(P.srec + (long long)(on ? pos : 0) * ROW_REC);
+      double2 e[5];
+#pragma unroll
+      for (int q = 0; q < 5; q++) e[q] = r[q];
+      const int pid = __double2hiint(e[4].y);
+      int rank = 0;
+      for (int q = 0; q < all; q++) rank += __shfl_sync(ALL, pid, q) < pid ? 1 : 0;
+      if (on) row_entry(e, l, x0, con + 6 * rank, s_x + rank);
+      __syncwarp();
+      row_accumulate(all, lane, n, cells, con, s_x, acc);
+      beg = end;
+    }
     // chunks of the merge: up to cap entries of each list; with entries left behind, only those
     // up to the smallest index T that ends a cut list are merged now
     while (__any_sync(ALL, beg < end)) {
@@ -167,8 +230,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) deposit_rows_kernel(const Part
       for (int e = lane; e < ROW_CHUNK; e += 32) {
         const bool on = e < total;
         int l = 0;
-#pragma unroll
-        for (int q = 1; q < 8; q++)  // the last list that begins at or before e
+        for (int q = 1; q < nl; q++)  // the last list that begins at or before e
           if (__shfl_sync(ALL, off, q) <= e) l = q;
         const int base = __shfl_sync(ALL, beg, l) - __shfl_sync(ALL, off, l);
         if (on) s_pid[e] = __double2hiint(P.srec[(long long)(base + e) * ROW_REC + 9]);
@@ -180,8 +242,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) deposit_rows_kernel(const Part
         const int pid = e < total ? s_pid[e] : 0x7fffffff;
         const bool on = e < total && pid <= T;
         int rank = 0, l = 0;
-#pragma unroll
-        for (int q = 0; q < 8; q++) {  // entries of list q below this one (its own: its position)
+        for (int q = 0; q < nl; q++) {  // entries of list q below this one (its own: its position)
           const int a = __shfl_sync(ALL, off, q), c = __shfl_sync(ALL, cnt, q);
           if (a <= e) l = q;
           if (!on) continue;
@@ -196,18 +257,8 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) deposit_rows_kernel(const Part
         const int base = __shfl_sync(ALL, beg, l) - __shfl_sync(ALL, off, l);
         if (on) {
           const double2* r = reinterpret_cast<const double2*>(P.srec + (long long)(base + e) * ROW_REC);
-          const double2 a = r[0], b = r[1], c = r[2], d = r[3], f = r[4];
-          const double wy = (l & 1) ? d.x : c.y;         // dyp : dym
-          const double wz = ((l >> 1) & 1) ? f.x : d.y;  // dzp : dzm
-          const double v0 = b.y * wy * wz, v1 = c.x * wy * wz;
-          double* o = con + 6 * rank;
-          o[0] = a.x * v0;
-          o[1] = a.x * v1;
-          o[2] = a.y * v0;
-          o[3] = a.y * v1;
-          o[4] = b.x * v0;
-          o[5] = b.x * v1;
-          s_x[rank] = __double2loint(f.y) - x0;
+          const double2 v[5] = {r[0], r[1], r[2], r[3], r[4]};
+          row_entry(v, l, x0, con + 6 * rank, s_x + rank);
         }
       }
       // how many entries of each list were merged: those up to T
@@ -223,22 +274,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) deposit_rows_kernel(const Part
       }
       const int merged = __reduce_add_sync(ALL, lane < 8 ? done : 0);
       __syncwarp();
-      // in particle order: lane 2 c + di adds component c to the corner di of the stencil
-      for (int e0 = 0; e0 < merged; e0 += 4) {
-        int cell[4];
-        double v[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-          const int e = min(e0 + q, merged - 1);
-          cell[q] = e0 + q < merged && lane < 6 ? s_x[e] - (lane & 1) : -1;
-          v[q] = con[6 * e + (lane < 6 ? lane : 0)];
-        }
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-          if (cell[q] >= 0 && cell[q] < n) acc[(lane >> 1) * cells + cell[q]] += v[q];
-          __syncwarp();
-        }
-      }
+      row_accumulate(merged, lane, n, cells, con, s_x, acc);
       beg += done;
     }
     for (int c = lane; c < n; c += 32) {

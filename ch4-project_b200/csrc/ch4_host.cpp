@@ -719,8 +719,12 @@ struct Engine : EngineBase {
   double* rec = nullptr;
   double* srec = nullptr;
   int* spid = nullptr;
-  int* row_start = nullptr;  // list starts of the deposit by rows
-  bool rows_ready = false;   // its records and keys are those of the state (the last sub-step wrote them)
+  // the deposit by rows: places drawn per list (and the cursor), ranges of the lists; by particle
+  // slot the place, by list the entries
+  int* row_count = nullptr;
+  int2* row_list = nullptr;
+  int2 *row_place = nullptr, *row_entry = nullptr;
+  bool rows_ready = false;  // its records and places are those of the state (the last sub-step wrote them)
   int2* crng = nullptr;   // {start, end} per home cell
   int* busy = nullptr;    // cells for the deposit merge pass, per gather block
   int *bcount = nullptr, *boff = nullptr, *dense = nullptr;
@@ -780,7 +784,8 @@ struct Engine : EngineBase {
     cudaFree(dbuf[0]);
     cudaFree(dbuf[1]);
     cudaFree(crng);
-    cudaFree(row_start);
+    cudaFree(row_count);
+    cudaFree(row_list);
     cudaFree(busy);
     cudaFree(bcount);
     cudaFree(boff);
@@ -818,6 +823,9 @@ struct Engine : EngineBase {
     cudaFree(rec);
     cudaFree(srec);
     cudaFree(spid);
+    cudaFree(row_place);
+    cudaFree(row_entry);
+    row_place = row_entry = nullptr;
     srec = nullptr;
     spid = nullptr;
     cudaFree(cubtmp);
@@ -900,8 +908,11 @@ struct Engine : EngineBase {
                                                                                     : 1;
     Q.nrec = nrec();
     Q.rows = by_rows();
-    Q.row_start = row_start;
     Q.rows_ready = rows_ready;
+    Q.row_place = row_place;
+    Q.row_count = row_count;
+    Q.row_list = row_list;
+    Q.row_entry = row_entry;
     Q.rec = rec;
     Q.srec = srec;
     Q.spid = spid;
@@ -1065,6 +1076,10 @@ struct Engine : EngineBase {
     if (n < 0 || (n > 0 && !parts)) return H->fail(CH4_ERR_ARG, "bad particle array");
     ch4_status st;
     if ((st = H->cuda(cudaStreamSynchronize(H->stream), "sync"))) return st;
+    if (rows_ready) {  // places drawn for a deposit that will not come
+      const size_t nb = row_bins(c.NX, c.NY, c.NZ);
+      if ((st = H->cuda(cudaMemset(row_count, 0, sizeof(int) * (nb + 1)), "row lists"))) return st;
+    }
     rows_ready = false;
     const bool sl = pslab();
     if (n != (sl ? np_all : np) || (sl && !mig)) {
@@ -1081,8 +1096,10 @@ struct Engine : EngineBase {
                     cudaMalloc(&order, sizeof(int) * n) == cudaSuccess &&
                     cudaMalloc(&order2, sizeof(int) * n) == cudaSuccess &&
                     (!twoway() || cudaMalloc(&rec, sizeof(double) * nrec() * (size_t)n) == cudaSuccess) &&
-                    (!twoway() || (cudaMalloc(&srec, sizeof(double) * nrec() * (size_t)n) == cudaSuccess &&
-                                   cudaMalloc(&spid, sizeof(int) * (size_t)n) == cudaSuccess));
+                    (!by_rows() || (cudaMalloc(&row_place, sizeof(int2) * (size_t)n) == cudaSuccess &&
+                                    cudaMalloc(&row_entry, sizeof(int2) * (size_t)n) == cudaSuccess)) &&
+                    (!twoway() || by_rows() || (cudaMalloc(&srec, sizeof(double) * nrec() * (size_t)n) == cudaSuccess &&
+                                                cudaMalloc(&spid, sizeof(int) * (size_t)n) == cudaSuccess));
           if (!ok) return H->fail(CH4_ERR_NOMEM, "sort buffers");
           if (rj_random() && (cudaMalloc(&rj_count, sizeof(int) * (size_t)n) != cudaSuccess ||
                               cudaMalloc(&rj_xz, 2 * sizeof(double) * (size_t)n) != cudaSuccess))
@@ -1401,8 +1418,11 @@ struct Engine : EngineBase {
       }
       const size_t nreg = (size_t)((c.NX + GATHER_BLOCK - 1) / GATHER_BLOCK) * c.NY * c.NZ;
       if (by_rows()) {
-        if (cudaMalloc(&row_start, sizeof(int) * ((size_t)row_bins(c.NX, c.NY, c.NZ) + 1)) != cudaSuccess)
+        const size_t nb = row_bins(c.NX, c.NY, c.NZ);
+        if (cudaMalloc(&row_count, sizeof(int) * (nb + 1)) != cudaSuccess ||
+            cudaMalloc(&row_list, sizeof(int2) * nb) != cudaSuccess)
           return H->fail(CH4_ERR_NOMEM, "row lists");
+        if (cudaMemset(row_count, 0, sizeof(int) * (nb + 1)) != cudaSuccess) return H->fail(CH4_ERR_CUDA, "row lists");
       } else if (cudaMalloc(&crng, sizeof(int2) * nhome()) != cudaSuccess ||
           cudaMalloc(&busy, sizeof(int) * nreg * GATHER_BLOCK) != cudaSuccess ||
           cudaMalloc(&dense, sizeof(int) * nreg * GATHER_BLOCK) != cudaSuccess ||
@@ -1843,8 +1863,8 @@ struct Engine : EngineBase {
               if (np > 0 && ++since_reorder >= REORDER_EVERY && (st = reorder_particles(1))) return st;
             } else {
               if ((st = H->cuda(launch_deposit(Q, key2, order2, cubtmp, bytes, H->stream), "deposit"))) return st;
-              // the deposit's sort already holds the slots in home-cell order
-              if (np > 0 && ++since_reorder >= REORDER_EVERY && (st = reorder_particles(0))) return st;
+              // (unless by rows, the deposit's sort already holds the slots in home-cell order)
+              if (np > 0 && ++since_reorder >= REORDER_EVERY && (st = reorder_particles(by_rows() ? 1 : 0))) return st;
             }
           } else if ((st = H->cuda(cudaMemsetAsync(dbuf[dcur_i], 0, dplanes() * N * sizeof(A), H->stream),
                                    "deposit zero"))) {

@@ -1,26 +1,30 @@
 // Two-way momentum deposit by lattice rows (included by particles.cuh inside namespace ch4).
 //
 // src/lagrange_feedback.c:11-256: the particle loop adds fac * fp * vol of every particle to
-// the 8 cells of its stencil.  Here the particles are radix-sorted (stably, laid out by
-// particle index) by the row segment their home cell lies in -- at most ROW_SEG cells of one
-// (y, z) row -- and one warp owns one segment of a lattice row: it merges the lists of the
-// four home rows around it in particle-index order and adds every particle to the two cells
-// it has in the row, in shared memory.  Each cell thus sums its particles in the reference's
-// order whatever the schedule, and no array runs over the home cells.
+// the 8 cells of its stencil.  Here every particle is listed under the row segment its home cell
+// lies in -- at most ROW_SEG cells of one (y, z) row -- and one warp owns one segment of a lattice
+// row: it merges the lists of the four home rows around it in particle-index order and adds
+// every particle to the two cells it has in the row, in shared memory.  Each cell thus sums its
+// particles in the reference's order whatever the schedule, and no array runs over the home
+// cells.
+//
+// The lists are built by counting: a particle draws its place in its list from a counter (the
+// sub-step that has just moved it does), a pass over the lists gives each its range, a pass over
+// the particles fills them in, and a last one puts every list in particle-index order -- the
+// order of the draws is the schedule's, the lists and sums are not.
 //
 // Why rows: at the workloads' 0.04 depositing particles per cell nearly every home cell is
 // empty, and a list per home cell (a range of 8 bytes each, cleared, filled, read and scanned
 // every step) moved more bytes than the particles; a row of 256 cells has some 10 particles a
-// list.  Keys are 8-10 bits shorter too, one to two radix passes less, and the records and keys
-// are written by the sub-step that has their inputs in registers.  Measured, us a step: 250,000
-// particles in 160^3 FP32 505 -> 431, 15,000 in 60x50x70 FP64 164 -> 109 (re-sort every 16 steps
-// and only of the planes that differ included).
+// list.  Measured, us a step, home cells -> rows: 250,000 particles in 160^3 FP32 505 -> 431,
+// 15,000 in 60x50x70 FP64 164 -> 109 (re-sort every 16 steps and only of the planes that differ
+// included); the lists by radix sort -> by counting: 390 -> 347 and 85 -> 53, 800,000 in 240^3
+// 1,155 -> 1,073 (four launches of the sort and the copy of the records into its order gone).
 #pragma once
 
 constexpr int ROW_SEG = 256;    // cells of a row that one warp owns
 constexpr int ROW_CHUNK = 64;   // merged entries in shared memory at a time (8 lists x 8)
 constexpr int ROW_WARPS = 4;    // warps per block
-constexpr int ROW_COPY = 64;    // records per block of row_lists_kernel, ROW_REC / 2 threads each
 constexpr int ROW_REC = 10;     // doubles of a record: fac*fp (3), dxm dxp dym dyp dzm dzp, {hx, index}
 
 // row segments along x: the last home cell (hx = NX) belongs to the last segment
@@ -35,7 +39,7 @@ __host__ __device__ __forceinline__ unsigned int row_bin(int hx, int hy, int hz,
 
 #ifdef __CUDACC__
 
-// Deposit record and row-segment key of one particle (src/lagrange_feedback.c:34-118).  The
+// Deposit record and place in its list of one particle (src/lagrange_feedback.c:34-118).  The
 // last sub-step of a step calls it with the state it has in registers; a and D (acceleration
 // and Du/Dt) are read from the state where `have` is not set.
 template <typename A>
@@ -52,10 +56,12 @@ __device__ __forceinline__ void deposit_rows_emit(const PartParams<A>& P, int ip
   const int o = P.pid[ip];
   const bool live = inside && (fac > 0.0) && beta != 0.0;
   const int hx = t.im + 1, hy = t.jm + 1, hz = t.km + 1;
-  const unsigned int nb = row_bins(P.NX, P.NY, P.NZ);
-  P.key[o] = (live ? 0u : nb) + row_bin(hx, hy, hz, P.NX, P.NY);
-  P.order[o] = ip;
-  if (!live) return;  // sorted after every list and never read
+  if (!live) {
+    P.row_place[ip] = make_int2(-1, 0);
+    return;
+  }
+  const int bin = (int)row_bin(hx, hy, hz, P.NX, P.NY);
+  P.row_place[ip] = make_int2(bin, atomicAdd(P.row_count + bin, 1));
   const double dr = pf[PF_DR * np + ip];
   double aa[3], DD[3];
   if (have) {
@@ -94,27 +100,69 @@ __global__ void deposit_rows_prepare_kernel(const PartParams<A> P) {
                     P.pf[CH4_PF(beta_coeff) * np + ip], false, (const double*)nullptr, (const double*)nullptr);
 }
 
-// The records of the depositing particles in sorted order (a list is then one run of them: no
-// load of the merge waits for an index), and start[b] = first sorted position with a key of at
-// least b, b = 0 .. nb; the blocks from `copies` on do the second.
-static __global__ void row_lists_kernel(const unsigned int* key, const int* slot, int n, unsigned int nb,
-                                        int copies, const double2* rec, double2* srec, int* start) {
+// the range of every list (bins of a warp together, at a place drawn from *cursor), the counters
+// cleared for the next sub-step
+static __global__ void row_ranges_kernel(int* count, unsigned int nb, int2* list, int* cursor) {
   grid_chain();
-  if ((int)blockIdx.x < copies) {
-    const int i = blockIdx.x * ROW_COPY + threadIdx.x / (ROW_REC / 2), part = threadIdx.x % (ROW_REC / 2);
-    if (i < n && key[i] < nb)
-      srec[(long long)i * (ROW_REC / 2) + part] = rec[(long long)slot[i] * (ROW_REC / 2) + part];
+  const unsigned int b = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  const int c = b < nb ? count[b] : 0;
+  int sum = c;  // inclusive prefix
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, sum, d);
+    if ((int)lane >= d) sum += v;
+  }
+  int base = 0;
+  if (lane == 31 && sum > 0) base = atomicAdd(cursor, sum);
+  base = __shfl_sync(0xffffffffu, base, 31) + sum - c;
+  if (b < nb) {
+    list[b] = make_int2(base, base + c);
+    if (c) count[b] = 0;
+  }
+}
+
+// the particles into their lists, as {index, slot}
+static __global__ void row_fill_kernel(const int2* place, const int2* list, const int* pid, int np, int2* entry,
+                                       int* cursor) {
+  grid_chain();
+  const int ip = blockIdx.x * blockDim.x + threadIdx.x;
+  if (ip == 0) *cursor = 0;  // for the next deposit
+  if (ip >= np) return;
+  const int2 p = place[ip];
+  if (p.x >= 0) entry[list[p.x].x + p.y] = make_int2(pid[ip], ip);
+}
+
+// every list in particle-index order, a warp per list: up to 32 entries ranked in registers, more
+// by a bitonic merge sort in place (for any length: an exchange with a partner beyond the end is
+// left out, as such a partner would be larger)
+static __global__ void row_order_kernel(const int2* list, unsigned int nb, int2* entry) {
+  grid_chain();
+  const unsigned int b = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
+  if (b >= nb) return;
+  const int2 l = list[b];
+  const int n = l.y - l.x;
+  if (n < 2) return;
+  int2* const e = entry + l.x;
+  if (n <= 32) {
+    const int2 v = (int)lane < n ? e[lane] : make_int2(0x7fffffff, 0);
+    int rank = 0;
+    for (int q = 0; q < n; q++) rank += __shfl_sync(0xffffffffu, v.x, q) < v.x ? 1 : 0;
+    if ((int)lane < n) e[rank] = v;
     return;
   }
-  const unsigned int b = (blockIdx.x - (unsigned)copies) * blockDim.x + threadIdx.x;
-  if (b > nb) return;
-  int lo = 0, hi = n;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (key[mid] < b) lo = mid + 1;
-    else hi = mid;
+  for (long long k = 2; k < 2LL * n; k <<= 1) {  // runs of k from runs of k / 2
+    for (long long j = k >> 1; j > 0; j >>= 1) {
+      // the first exchange of a merge mirrors the second run, the others are at distance j
+      for (long long i = lane; i < n; i += 32) {
+        const long long q = j == k >> 1 ? (i | (k - 1)) - (i & (k - 1)) : i ^ j;
+        if (q > i && q < n) {
+          const int2 a = e[i], c = e[q];
+          if (a.x > c.x) e[i] = c, e[q] = a;
+        }
+      }
+      __syncwarp();
+    }
   }
-  start[b] = lo;
 }
 
 // shared memory of one warp: the contributions by merged position (component c of corner di
@@ -180,8 +228,9 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) deposit_rows_kernel(const Part
   if (lane < 8 && (lane < 4 || seg + 1 < ns)) {
     const unsigned int b = ((unsigned)(k + ((lane >> 1) & 1)) * (unsigned)(P.NY + 1) + (unsigned)(j + (lane & 1))) *
                                (unsigned)ns + (unsigned)(seg + (lane >> 2));
-    beg = P.row_start[b];
-    end = P.row_start[b + 1];
+    const int2 range = P.row_list[b];
+    beg = range.x;
+    end = range.y;
   }
   constexpr unsigned ALL = 0xffffffffu;
   if (__any_sync(ALL, beg < end)) {
@@ -201,11 +250,12 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) deposit_rows_kernel(const Part
         if (__shfl_sync(ALL, off, q) <= lane) l = q;
       const int pos = __shfl_sync(ALL, beg, l) - __shfl_sync(ALL, off, l) + lane;
       const bool on = lane < all;
-      const double2* r = reinterpret_cast<const double2*>(P.srec + (long long)(on ? pos : 0) * ROW_REC);
+      const int2 who = on ? P.row_entry[pos] : make_int2(0x7fffffff, 0);
+      const double2* r = reinterpret_cast<const double2*>(P.rec + (long long)who.y * ROW_REC);
       double2 e[5];
 #pragma unroll
       for (int q = 0; q < 5; q++) e[q] = r[q];
-      const int pid = __double2hiint(e[4].y);
+      const int pid = who.x;
       int rank = 0;
       for (int q = 0; q < all; q++) rank += __shfl_sync(ALL, pid, q) < pid ? 1 : 0;
       if (on) row_entry(e, l, x0, con + 6 * rank, s_x + rank);
@@ -233,7 +283,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) deposit_rows_kernel(const Part
         for (int q = 1; q < nl; q++)  // the last list that begins at or before e
           if (__shfl_sync(ALL, off, q) <= e) l = q;
         const int base = __shfl_sync(ALL, beg, l) - __shfl_sync(ALL, off, l);
-        if (on) s_pid[e] = __double2hiint(P.srec[(long long)(base + e) * ROW_REC + 9]);
+        if (on) s_pid[e] = P.row_entry[base + e].x;
       }
       __syncwarp();
       const bool cut = lane < 8 && end - beg > cnt;
@@ -256,7 +306,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) deposit_rows_kernel(const Part
         }
         const int base = __shfl_sync(ALL, beg, l) - __shfl_sync(ALL, off, l);
         if (on) {
-          const double2* r = reinterpret_cast<const double2*>(P.srec + (long long)(base + e) * ROW_REC);
+          const double2* r = reinterpret_cast<const double2*>(P.rec + (long long)P.row_entry[base + e].y * ROW_REC);
           const double2 v[5] = {r[0], r[1], r[2], r[3], r[4]};
           row_entry(v, l, x0, con + 6 * rank, s_x + rank);
         }

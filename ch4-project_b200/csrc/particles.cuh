@@ -86,9 +86,12 @@ struct PartParams {
   // trilinear momentum deposit by lattice rows (deposit_rows.cuh): rec then holds ROW_REC
   // doubles per state slot, one record after the other
   int rows;
-  int rows_ready;        // the last sub-step wrote the records and keys
+  int rows_ready;        // the last sub-step wrote the records and places
   int emit;              // this sub-step writes them
-  int* row_start;        // [row_bins + 1] first sorted position of every row segment's list
+  int2* row_place;       // [np] by slot: list and place in it (-1: deposits nothing)
+  int* row_count;        // [row_bins] places drawn, then the cursor that the lists' ranges are drawn from
+  int2* row_list;        // [row_bins] first entry and end of every list
+  int2* row_entry;       // [np] {index, slot} by list
   double* srec;          // [nrec][np] the same by sorted position (depositing particles only)
   int* spid;             // particle index by sorted position
   int2* cell_rng;        // [(NX+1)(NY+1)(NZ+1)] {start, end} of every home cell's sorted run

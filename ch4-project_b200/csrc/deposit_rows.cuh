@@ -167,14 +167,15 @@ static __global__ void row_order_kernel(const int2* list, unsigned int nb, int2*
 
 // shared memory of one warp: the contributions by merged position (component c of corner di
 // at 2 c + di), the row's sums (three rows of `cells`), indices and cells of the merged entries
-__host__ __device__ __forceinline__ int row_cells(int NX) { return NX < ROW_SEG ? (NX + 1) & ~1 : ROW_SEG; }
+__host__ __device__ __forceinline__ int row_cells(int NX) { return (NX < ROW_SEG ? NX : ROW_SEG) + 1; }  // and a spare one
 __host__ __device__ __forceinline__ int row_shared(int NX) {
-  return ROW_CHUNK * 6 * 8 + 3 * row_cells(NX) * 8 + ROW_CHUNK * 2 * 4;
+  return ROW_CHUNK * 6 * 8 + 3 * row_cells(NX) * 8 + ROW_CHUNK * 3 * 4;
 }
 
-// what a record of list l adds to the two cells it has in the row: component c of corner di at
-// o[2 c + di]; *x: the cell of corner 0 (corner 1: the one before)
-__device__ __forceinline__ void row_entry(const double2* r, int l, int x0, double* o, int* x) {
+// what a record of list l adds to the two cells it has in the row of n cells: component c of
+// corner di at o[2 c + di], its cell (the one of corner 1 comes before) at at[di]; a cell outside
+// the row is `spare`, which is never read
+__device__ __forceinline__ void row_entry(const double2* r, int l, int x0, int n, int spare, double* o, int* at) {
   const double wy = (l & 1) ? r[3].x : r[2].y;         // dyp : dym
   const double wz = ((l >> 1) & 1) ? r[4].x : r[3].y;  // dzp : dzm
   const double v0 = r[1].y * wy * wz, v1 = r[2].x * wy * wz;
@@ -184,27 +185,25 @@ __device__ __forceinline__ void row_entry(const double2* r, int l, int x0, doubl
   o[3] = r[0].y * v1;
   o[4] = r[1].x * v0;
   o[5] = r[1].x * v1;
-  *x = __double2loint(r[4].y) - x0;
+  const unsigned int c0 = (unsigned)(__double2loint(r[4].y) - x0), c1 = c0 - 1u;
+  at[0] = c0 < (unsigned)n ? (int)c0 : spare;
+  at[1] = c1 < (unsigned)n ? (int)c1 : spare;
 }
 
 // the merged entries in particle order: lane 2 c + di adds component c to the corner di
-__device__ __forceinline__ void row_accumulate(int merged, int lane, int n, int cells, const double* con,
-                                               const int* s_x, double* acc) {
-  for (int e0 = 0; e0 < merged; e0 += 4) {
-    int cell[4];
-    double v[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int e = min(e0 + q, merged - 1);
-      cell[q] = e0 + q < merged && lane < 6 ? s_x[e] - (lane & 1) : -1;
-      v[q] = con[6 * e + (lane < 6 ? lane : 0)];
-    }
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      if (cell[q] >= 0 && cell[q] < n) acc[(lane >> 1) * cells + cell[q]] += v[q];
-      __syncwarp();
+__device__ __forceinline__ void row_accumulate(int merged, int lane, int cells, const double* con, const int* s_at,
+                                               double* acc) {
+  if (lane < 6) {
+    double* const mine = acc + (lane >> 1) * cells;
+    const int* at = s_at + (lane & 1);
+    const double* v = con + lane;
+#pragma unroll 4
+    for (int e = 0; e < merged; e++) {
+      mine[at[2 * e]] += v[6 * e];
+      __syncwarp(0x3f);
     }
   }
+  __syncwarp();
 }
 
 template <typename A>
@@ -215,7 +214,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) deposit_rows_kernel(const Part
   double* const con = row_smem + warp * (row_shared(P.NX) / 8);
   double* const acc = con + ROW_CHUNK * 6;
   int* const s_pid = reinterpret_cast<int*>(acc + 3 * cells);
-  int* const s_x = s_pid + ROW_CHUNK;
+  int* const s_at = s_pid + ROW_CHUNK;
   const int ns = row_segs(P.NX), nl = ns == 1 ? 4 : 8;  // lists
   const unsigned int w = blockIdx.x * ROW_WARPS + warp;  // of plane k's ns * NY
   const int j = (int)(ns == 1 ? w : w / (unsigned)ns), seg = (int)w - j * ns, k = blockIdx.y;
@@ -258,9 +257,9 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) deposit_rows_kernel(const Part
       const int pid = who.x;
       int rank = 0;
       for (int q = 0; q < all; q++) rank += __shfl_sync(ALL, pid, q) < pid ? 1 : 0;
-      if (on) row_entry(e, l, x0, con + 6 * rank, s_x + rank);
+      if (on) row_entry(e, l, x0, n, cells - 1, con + 6 * rank, s_at + 2 * rank);
       __syncwarp();
-      row_accumulate(all, lane, n, cells, con, s_x, acc);
+      row_accumulate(all, lane, cells, con, s_at, acc);
       beg = end;
     }
     // chunks of the merge: up to cap entries of each list; with entries left behind, only those
@@ -308,7 +307,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) deposit_rows_kernel(const Part
         if (on) {
           const double2* r = reinterpret_cast<const double2*>(P.rec + (long long)P.row_entry[base + e].y * ROW_REC);
           const double2 v[5] = {r[0], r[1], r[2], r[3], r[4]};
-          row_entry(v, l, x0, con + 6 * rank, s_x + rank);
+          row_entry(v, l, x0, n, cells - 1, con + 6 * rank, s_at + 2 * rank);
         }
       }
       // how many entries of each list were merged: those up to T
@@ -324,7 +323,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) deposit_rows_kernel(const Part
       }
       const int merged = __reduce_add_sync(ALL, lane < 8 ? done : 0);
       __syncwarp();
-      row_accumulate(merged, lane, n, cells, con, s_x, acc);
+      row_accumulate(merged, lane, cells, con, s_at, acc);
       beg += done;
     }
     for (int c = lane; c < n; c += 32) {

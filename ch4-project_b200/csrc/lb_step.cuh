@@ -552,7 +552,7 @@ __device__ __forceinline__ void lb_cell(const StepParams<A>& P, int x, int y, in
       rho = mom0(f);
     }
     tl = les_tau<EXACT>(P, x, y, z, idx, f, rho, ul[0], ul[1], ul[2], u2);
-    P.tau_les[idx] = tl;
+    if (P.feat & K_LSTRAIN) P.tau_les[idx] = tl;  // the only reader: the stress form, next step
   }
   constexpr int sets = 1 + (THERM ? 1 : 0) + (SCAL ? 1 : 0);
   const S* p = pop_at<S>(P.fin[0], sets * Q * POP_BLOCK, idx);

@@ -8,14 +8,15 @@
 // wrap of sendrecv_particles (src/lagrange.c:4028-4221), fused per particle.
 //
 // Two-way momentum deposit (src/lagrange_feedback.c:11-256) as a deterministic
-// gather: particles are stably radix-sorted by their home cell (the lower corner
+// gather: by lattice rows (deposit_rows.cuh), or for z-slabs, the tricubic stencil and the
+// heat deposit by home cells: particles are stably radix-sorted by their home cell (the lower corner
 // of the trilinear stencil, shifted by +1 so that the halo row -1 is index 0);
 // every lattice cell then merges the (up to 8) home-cell lists around it in
 // particle-index order, which is exactly the order in which the reference's
 // particle loop adds to that cell.  Deposits on halo cells are dropped as in the
 // reference's border fold (src/lagrange_feedback.c:525-835).
 //
-// Spatial order: the state slots are kept sorted by home cell (re-sorted every few
+// Spatial order: the state slots are kept sorted by home cell (re-sorted every sixteen
 // steps), so that the particles of one warp read neighbouring lattice rows in the
 // interpolation and neighbouring records in the gather.  pid[slot] is the particle's
 // index in the caller's array: the sort input is laid out in that index order, so

@@ -219,7 +219,9 @@ class Simulation:
         self._check(lib().ch4_set_particles(self.h, parts, len(parts)), "set_particles")
 
     def get_particles(self, n):
-        arr = (Particle * n)()
+        kind = Particle * n
+        # every entry is written, except those that a z-slab does not hold: only there zeroed
+        arr = kind() if n == 0 or self.cfg.nz_global > 0 else kind.from_buffer(np.empty(C.sizeof(kind), np.uint8))
         self._check(lib().ch4_get_particles(self.h, arr, n), "get_particles")
         return arr
 

@@ -124,6 +124,8 @@ cudaError_t launch_ghosts_in(const PartParams<double>& P, const double* from_dow
 cudaError_t launch_ghosts_in(const PartParams<float>& P, const double* from_down, const double* from_up, int cap,
                              cudaStream_t st);
 
+// records (ch4_particle) of the state slots s0 .. s0 + m - 1 of np
+cudaError_t launch_particle_records(const double* pf, int np, int s0, int m, double* out, cudaStream_t st);
 // Lagrangian averages per particle type (dump_particle_averages): partial holds
 // types * 3 * nblk * 11 * 2 doubles, out_dev receives [types][CH4_PART_AVG_FIELDS]
 cudaError_t launch_particle_averages(const double* pf, int np, int types, double* partial, int nblk, double* out_dev,

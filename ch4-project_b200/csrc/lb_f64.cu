@@ -7,6 +7,7 @@
 #include "lb_kernels.cuh"
 #include "lb_launch.inc"
 #include "part_avg.cuh"
+#include "part_records.cuh"
 
 namespace ch4 {
 
@@ -67,6 +68,11 @@ cudaError_t launch_aos_to_soa(const StepParams<double>& P, LaunchShape, int set,
 cudaError_t launch_soa_to_aos(const StepParams<double>& P, LaunchShape, int set, const void* soa, double* aos, int z0,
                               int nz, cudaStream_t st) {
   return s2a_t<double, double>(P, set, soa, aos, z0, nz, st);
+}
+cudaError_t launch_particle_records(const double* pf, int np, int s0, int m, double* out, cudaStream_t st) {
+  if (m <= 0) return cudaSuccess;
+  particle_records_kernel<<<(m + PREC_SLOTS - 1) / PREC_SLOTS, PREC_THREADS, 0, st>>>(pf, np, s0, m, out);
+  return cudaGetLastError();
 }
 cudaError_t launch_particle_averages(const double* pf, int np, int types, double* partial, int nblk, double* out_dev,
                                      cudaStream_t st) {

@@ -661,6 +661,7 @@ struct Engine : EngineBase {
   A* staging_d2 = nullptr;
   A* staging_h2 = nullptr;
   size_t staging_bytes = 0, hit_h_bytes = 0;
+  std::recursive_mutex staging_mu;  // read-backs and uploads from several threads share the buffers
   // particle records pass through the halves of the staging buffer, at most PART_CHUNK bytes
   // at a time; a small lattice's buffer is widened to PART_STAGING for them
   static constexpr size_t PART_STAGING = 1u << 20, PART_CHUNK = 16u << 20;
@@ -1360,6 +1361,7 @@ struct Engine : EngineBase {
 
   int particle_count() const override { return np; }
   ch4_status get_particles(ch4_particle* parts, int n) override {
+    std::lock_guard<std::recursive_mutex> hold(staging_mu);
     // a z-slab fills the entries of the particles it holds in an array of all of them
     const int lim = pslab() ? np_all : np;
     if (n < 0 || (n > 0 && !parts)) return H->fail(CH4_ERR_ARG, "bad particle array");
@@ -1622,6 +1624,7 @@ struct Engine : EngineBase {
   }
 
   ch4_status set_pop(int set, const double* aos, int brd) override {
+    std::lock_guard<std::recursive_mutex> hold(staging_mu);
     upart_current = false;
     if (!nsets_on[set]) return H->fail(CH4_ERR_ARG, "population set %d is not enabled", set);
     H->initialized = false;
@@ -1630,6 +1633,7 @@ struct Engine : EngineBase {
   }
 
   ch4_status get_pop(int set, double* aos, int brd) override {
+    std::lock_guard<std::recursive_mutex> hold(staging_mu);
     if (ch4_status rs = ready()) return rs;
     if (!nsets_on[set]) return H->fail(CH4_ERR_ARG, "population set %d is not enabled", set);
     const size_t row = (size_t)c.NX * NPOP;
@@ -1960,6 +1964,7 @@ struct Engine : EngineBase {
   }
 
   ch4_status fields(double* dens, double* u, double* t, double* s, double* force, int brd) override {
+    std::lock_guard<std::recursive_mutex> hold(staging_mu);
     if (ch4_status rs = ready()) return rs;
     bind_pops(cur);
     ch4_status st;
@@ -3710,6 +3715,7 @@ struct ch4_ensemble {
   float *fields_d = nullptr, *fields_h = nullptr;
   size_t fields_bytes = 0;
   cudaEvent_t fields_ev[2] = {nullptr, nullptr};
+  std::mutex fields_mu;  // slots read by several threads
 
   static size_t fields_need(const Slot& s) {
     return (size_t)s.N * (4 + s.nsets_on[1] + s.nsets_on[2]) * sizeof(float);
@@ -3740,6 +3746,7 @@ struct ch4_ensemble {
     return CH4_OK;
   }
   ch4_status fields_direct(const Slot& s, double* dens, double* u, double* t, double* sc) {
+    std::lock_guard<std::mutex> hold(fields_mu);
     const size_t n1 = (size_t)s.N, plane = (size_t)s.cfg.NX * s.cfg.NY;
     const int want = (dens ? 1 : 0) | (u ? 2 : 0) | (t && s.nsets_on[1] ? 4 : 0) | (sc && s.nsets_on[2] ? 8 : 0);
     if (t && !s.nsets_on[1]) std::fill(t, t + n1, 0.0);

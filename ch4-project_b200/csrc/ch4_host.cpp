@@ -1082,7 +1082,7 @@ struct Engine : EngineBase {
     if ((st = H->cuda(cudaStreamSynchronize(H->stream), "sync"))) return st;
     if (rows_ready) {  // places drawn for a deposit that will not come
       const size_t nb = row_bins(c.NX, c.NY, c.NZ);
-      if ((st = H->cuda(cudaMemset(row_count, 0, sizeof(int) * (nb + 1)), "row lists"))) return st;
+      if ((st = H->cuda(cudaMemsetAsync(row_count, 0, sizeof(int) * (nb + 1), H->stream), "row lists"))) return st;
     }
     rows_ready = false;
     const bool sl = pslab();
@@ -1132,7 +1132,7 @@ struct Engine : EngineBase {
       }
       np = n;
     }
-    if ((st = H->cuda(cudaMemset(pstatus, 0, sizeof(int)), "particle status"))) return st;
+    if ((st = H->cuda(cudaMemsetAsync(pstatus, 0, sizeof(int), H->stream), "particle status"))) return st;
     if (n == 0) return CH4_OK;
     for (int i = 0; i < n; i++)
       if (!std::isfinite(parts[i].x) || !std::isfinite(parts[i].y) || !std::isfinite(parts[i].z))
@@ -1166,13 +1166,14 @@ struct Engine : EngineBase {
       }
     }
     if (n > 0 &&
-        ((st = H->cuda(cudaMemcpy(pf, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice), "particles up")) ||
-         (st = H->cuda(cudaMemcpy(pf_alt, pf, sizeof(double) * h.size(), cudaMemcpyDeviceToDevice), "particles up"))))
+        ((st = upload(pf, h.data(), sizeof(double) * h.size(), "particles up")) ||
+         (st = H->cuda(cudaMemcpyAsync(pf_alt, pf, sizeof(double) * h.size(), cudaMemcpyDeviceToDevice, H->stream),
+                       "particles up"))))
       return st;
     find_planes(h, n);
     since_reorder = REORDER_EVERY;  // sort at the first opportunity
     if (n == 0) return CH4_OK;
-    return H->cuda(cudaMemcpy(pid, ids.data(), sizeof(int) * n, cudaMemcpyHostToDevice), "particle ids up");
+    return upload(pid, ids.data(), sizeof(int) * n, "particle ids up");
   }
 
   // z-slab: u^{n+1} of the two planes next to each face to the neighbours, theirs into the
@@ -1422,6 +1423,14 @@ struct Engine : EngineBase {
     return b;
   }
 
+  // host memory -> device, finished on return.  On the handle's stream, as the clears: the legacy
+  // stream is not ordered with it, and neither a clear nor the end of a copy from pageable memory
+  // has to be over when the call returns.
+  ch4_status upload(void* d, const void* s, size_t bytes, const char* what) {
+    const ch4_status st = H->cuda(cudaMemcpyAsync(d, s, bytes, cudaMemcpyHostToDevice, H->stream), what);
+    return st ? st : H->cuda(cudaStreamSynchronize(H->stream), what);
+  }
+
   ch4_status alloc() override {
     for (int b = 0; b < 2; b++) {
       const cudaError_t e = cudaMalloc(&f[0][b], pop_values(N, sets()) * sbytes);
@@ -1435,12 +1444,12 @@ struct Engine : EngineBase {
       return H->fail(CH4_ERR_NOMEM, "u for particles");
     if (lagr()) {
       if (cudaMalloc(&pstatus, sizeof(int)) != cudaSuccess) return H->fail(CH4_ERR_NOMEM, "particle status");
-      if (cudaMemset(pstatus, 0, sizeof(int)) != cudaSuccess) return H->fail(CH4_ERR_CUDA, "particle status");
+      if (cudaMemsetAsync(pstatus, 0, sizeof(int), H->stream) != cudaSuccess) return H->fail(CH4_ERR_CUDA, "particle status");
     }
     if (twoway()) {
       for (int b = 0; b < 2; b++) {
         if (cudaMalloc(&dbuf[b], dplanes() * N * sizeof(A)) != cudaSuccess) return H->fail(CH4_ERR_NOMEM, "deposit");
-        if (cudaMemset(dbuf[b], 0, dplanes() * N * sizeof(A)) != cudaSuccess)
+        if (cudaMemsetAsync(dbuf[b], 0, dplanes() * N * sizeof(A), H->stream) != cudaSuccess)
           return H->fail(CH4_ERR_CUDA, "deposit memset");
       }
       const size_t nreg = (size_t)((c.NX + GATHER_BLOCK - 1) / GATHER_BLOCK) * c.NY * c.NZ;
@@ -1449,7 +1458,8 @@ struct Engine : EngineBase {
         if (cudaMalloc(&row_count, sizeof(int) * (nb + 1)) != cudaSuccess ||
             cudaMalloc(&row_list, sizeof(int2) * nb) != cudaSuccess)
           return H->fail(CH4_ERR_NOMEM, "row lists");
-        if (cudaMemset(row_count, 0, sizeof(int) * (nb + 1)) != cudaSuccess) return H->fail(CH4_ERR_CUDA, "row lists");
+        if (cudaMemsetAsync(row_count, 0, sizeof(int) * (nb + 1), H->stream) != cudaSuccess)
+          return H->fail(CH4_ERR_CUDA, "row lists");
       } else if (cudaMalloc(&crng, sizeof(int2) * nhome()) != cudaSuccess ||
           cudaMalloc(&busy, sizeof(int) * nreg * GATHER_BLOCK) != cudaSuccess ||
           cudaMalloc(&dense, sizeof(int) * nreg * GATHER_BLOCK) != cudaSuccess ||
@@ -1466,8 +1476,7 @@ struct Engine : EngineBase {
       if (cudaMalloc(&fmbuf, sizeof init) != cudaSuccess ||
           cudaMalloc(&fmpart, sizeof(double) * FM_SUMS * 2 * (size_t)fm_nblocks) != cudaSuccess)
         return H->fail(CH4_ERR_NOMEM, "force corrections");
-      if (cudaMemcpy(fmbuf, init, sizeof init, cudaMemcpyHostToDevice) != cudaSuccess)
-        return H->fail(CH4_ERR_CUDA, "force corrections");
+      if (ch4_status e = upload(fmbuf, init, sizeof init, "force corrections")) return e;
     }
     if (c.flags & CH4_F_FLUID_LES) {
       if (cudaMalloc(&ules, 4 * N * sizeof(A)) != cudaSuccess) return H->fail(CH4_ERR_NOMEM, "ules");
@@ -1488,8 +1497,7 @@ struct Engine : EngineBase {
           t[j] = (A)std::pow(C * 1.0, 2.0);
         }
         if (cudaMalloc(&vd, c.NY * sizeof(A)) != cudaSuccess) return H->fail(CH4_ERR_NOMEM, "van Driest table");
-        if (cudaMemcpy(vd, t.data(), c.NY * sizeof(A), cudaMemcpyHostToDevice) != cudaSuccess)
-          return H->fail(CH4_ERR_CUDA, "van Driest table");
+        if (ch4_status e = upload(vd, t.data(), c.NY * sizeof(A), "van Driest table")) return e;
       }
     }
     const int nk = 2 * c.NY + c.NX;
@@ -1533,7 +1541,7 @@ struct Engine : EngineBase {
         double x = (double)i + 0.5;
         t[c.NY + i] = (A)(c.Amp_y * fnx * std::sin(kn * 2 * 3.14159265359 * x / LX));
       }
-      if ((st = H->cuda(cudaMemcpy(kol, t.data(), nk * sizeof(A), cudaMemcpyHostToDevice), "kol upload"))) return st;
+      if ((st = upload(kol, t.data(), nk * sizeof(A), "kol upload"))) return st;
     }
     return CH4_OK;
   }
@@ -4019,7 +4027,9 @@ ch4_status ch4_ensemble_add(ch4_ensemble* E, const ch4_config* cfg, int* slot) {
     }
     for (int i = 0; i < cfg->NX; i++)
       t[cfg->NY + i] = (float)(cfg->Amp_y * fnx * std::sin(kn * 2 * 3.14159265359 * ((double)i + 0.5) / LX));
-    if ((st = E->cuda(cudaMemcpy(s.kol, t.data(), nk * sizeof(float), cudaMemcpyHostToDevice), "kol"))) return st;
+    if ((st = E->cuda(cudaMemcpyAsync(s.kol, t.data(), nk * sizeof(float), cudaMemcpyHostToDevice, E->stream), "kol")) ||
+        (st = E->cuda(cudaStreamSynchronize(E->stream), "kol")))
+      return st;
   }
   // rest state p = w, g = h = 0
   std::vector<double> rest((size_t)s.N * NPOP);

@@ -1,0 +1,105 @@
+"""The host code of the library (csrc/ch4_host.cpp) over a faked CUDA runtime and faked kernel
+launchers (host_fakes.cpp): what it launches, in which order, and what it leaves behind when a
+call fails.  No GPU; the failures are error codes that a fake returns."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from ch4b200 import abi
+from lbcases import make_case
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+REPO = os.path.dirname(HERE)
+CUDA_INC = "/usr/local/cuda/include"
+
+if not os.path.exists(os.path.join(CUDA_INC, "cuda_runtime.h")):
+    pytest.skip("no CUDA headers", allow_module_level=True)
+
+
+@pytest.fixture(scope="module")
+def fakes(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("fakes") / "libfakes.so")
+    csrc = os.path.join(REPO, "ch4-project_b200", "csrc")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I", CUDA_INC, "-I", csrc,
+                    os.path.join(csrc, "ch4_host.cpp"), os.path.join(csrc, "h5file.cpp"),
+                    os.path.join(HERE, "host_fakes.cpp"), "-o", so], check=True)
+    L = C.CDLL(so)
+    L.fake_log.restype = L.fake_faults.restype = C.c_char_p
+    return L
+
+
+class Handle:
+    """A handle of the faked library holding a case's populations and particles."""
+
+    def __init__(self, L, cfg, state):
+        self.L, self.h, self.cfg = L, C.c_void_p(), cfg
+        L.fake_reset()
+        assert L.ch4_create(C.byref(cfg), C.byref(self.h)) == 0
+        for k in ("p", "g", "h"):
+            if k in state:
+                a = np.ascontiguousarray(state[k])
+                assert L.ch4_set_pop(self.h, C.c_char(k.encode()), a.ctypes.data_as(C.c_void_p), 0) == 0
+
+    def set_particles(self, parts):
+        assert self.L.ch4_set_particles(self.h, parts, len(parts)) == 0
+
+    def initialize(self):
+        assert self.L.ch4_initialize(self.h) == 0
+
+    def step(self, n=1):
+        return self.L.ch4_step(self.h, n)
+
+    def log(self):
+        out = self.L.fake_log().decode().split("\n")[:-1]
+        faults = self.L.fake_faults().decode()
+        self.L.fake_reset()
+        assert faults == ""
+        return out
+
+    def close(self):
+        self.L.ch4_destroy(self.h)
+
+
+@pytest.fixture
+def handle(fakes):
+    made = []
+
+    def make(name, **over):
+        _, cfg, state = make_case(name, seed=1, **over)
+        made.append(Handle(fakes, cfg, state))
+        return made[-1], state
+
+    yield make
+    for h in made:
+        h.close()
+
+
+@pytest.mark.parametrize("name", ["kolmogorov", "les_vd", "cpower", "particles", "particles_tc"])
+def test_uploads_are_ordered_with_the_steps(handle, name):
+    """Every table, clear and upload is ordered with the first launch that may read it."""
+    h, state = handle(name)
+    if "part" in state:
+        h.set_particles(state["part"])
+    h.initialize()
+    assert h.step(3) == 0
+    if "part" in state:
+        h.set_particles(state["part"])
+        assert h.step(2) == 0
+        h.set_particles((abi.Particle * 0)())
+        assert h.step(2) == 0
+    h.log()
+
+
+def test_ensemble_tables_are_ordered_with_the_steps(fakes):
+    _, cfg, state = make_case("kolmogorov", seed=1)
+    fakes.fake_reset()
+    ens, slot = C.c_void_p(), C.c_int()
+    assert fakes.ch4_ensemble_create(abi.STORE_F32, C.c_size_t(1 << 30), C.byref(ens)) == 0
+    assert fakes.ch4_ensemble_add(ens, C.byref(cfg), C.byref(slot)) == 0
+    assert fakes.ch4_ensemble_initialize(ens, slot) == 0
+    assert fakes.ch4_ensemble_step(ens, 3) == 0
+    assert fakes.fake_faults().decode() == ""
+    fakes.ch4_ensemble_destroy(ens)

@@ -1125,7 +1125,7 @@ struct Engine : EngineBase {
           np = n;
           PartParams<A> Q = part_params();
           size_t bytes = 0;
-          if ((st = H->cuda(launch_deposit(Q, key2, order2, nullptr, bytes, H->stream), "sort size"))) return st;
+          if ((st = H->cuda(launch_deposit_scratch(Q, key2, order2, bytes), "sort size"))) return st;
           cubbytes = bytes;
           if (cudaMalloc(&cubtmp, bytes ? bytes : 16) != cudaSuccess) return H->fail(CH4_ERR_NOMEM, "sort scratch");
         }

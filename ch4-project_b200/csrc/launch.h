@@ -106,8 +106,11 @@ cudaError_t launch_particle_arrive(const PartParams<float>& P, const int* keep, 
 // that re-entered in the last sub-step
 cudaError_t launch_particle_reinject(const PartParams<double>& P, const double* xz, cudaStream_t st);
 cudaError_t launch_particle_reinject(const PartParams<float>& P, const double* xz, cudaStream_t st);
-// two-way deposit into P.dep; `tmp`/`tmp_bytes` is CUB scratch (query with tmp == nullptr),
-// key2/order2 are the sort's output buffers
+// scratch that the deposit and the re-sort of P's particles need
+cudaError_t launch_deposit_scratch(const PartParams<double>& P, unsigned int* key2, int* order2, size_t& bytes);
+cudaError_t launch_deposit_scratch(const PartParams<float>& P, unsigned int* key2, int* order2, size_t& bytes);
+// two-way deposit into P.dep (zeros where there are no particles); `tmp`/`tmp_bytes` is that
+// scratch, key2/order2 are the sort's output buffers
 // (stage 0: all; 1: the keys and records of the slab's own particles; 2: the sort and gather)
 cudaError_t launch_deposit(const PartParams<double>& P, unsigned int* key2, int* order2, void* tmp, size_t& tmp_bytes,
                            cudaStream_t st, int stage = 0);

@@ -60,6 +60,9 @@ cudaError_t launch_particle_arrive(const PartParams<float>& P, const int* keep, 
                                    int nd, const double* from_up, int nu, cudaStream_t st) {
   return arrive_t<float>(P, keep, nkeep, from_down, nd, from_up, nu, st);
 }
+cudaError_t launch_deposit_scratch(const PartParams<float>& P, unsigned int* key2, int* order2, size_t& bytes) {
+  return deposit_scratch_t<float>(P, key2, order2, bytes);
+}
 cudaError_t launch_deposit(const PartParams<float>& P, unsigned int* key2, int* order2, void* tmp, size_t& tmp_bytes,
                            cudaStream_t st, int stage) {
   return deposit_t<float>(P, key2, order2, tmp, tmp_bytes, st, stage);

@@ -148,8 +148,11 @@ using S = cudaStream_t;
   cudaError_t launch_particle_reinject(const PartParams<A>&, const double*, S st) {                                    \
     return launched("launch_particle_reinject", st);                                                                   \
   }                                                                                                                    \
-  cudaError_t launch_deposit(const PartParams<A>& P, unsigned int*, int*, void* tmp, size_t& bytes, S st, int stage) { \
-    if (!tmp) bytes = 64;                                                                                              \
+  cudaError_t launch_deposit_scratch(const PartParams<A>&, unsigned int*, int*, size_t& bytes) {                       \
+    return bytes = 64, cudaSuccess;                                                                                    \
+  }                                                                                                                    \
+  cudaError_t launch_deposit(const PartParams<A>& P, unsigned int*, int*, void* tmp, size_t&, S st, int stage) {       \
+    if (P.nsort > 0) need("launch_deposit", tmp);                                                                      \
     return launched("launch_deposit", st, "stage " + std::to_string(stage) + (P.rows_ready ? " ready" : ""));          \
   }                                                                                                                    \
   cudaError_t launch_ghosts_out(const PartParams<A>&, double* down, double* up, int, int* counts, S st) {              \

@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 import oracle as O
+from ch4b200 import abi
 from lbcases import make_case, make_particles, run_restatement
 
 pytestmark = pytest.mark.gpu
@@ -70,3 +71,25 @@ def test_rows_f32_reproducible(name):
     a, b = run(cfg, state, parts, c["steps"]), run(cfg, state, parts, c["steps"])
     assert np.array_equal(a[0], b[0])
     assert all(np.array_equal(a[1][k], b[1][k]) for k in a[1])
+
+
+@pytest.mark.parametrize("name", ["particles", "particles_tc", "particles_tt"])
+def test_nothing_deposits_once_the_particles_are_removed(name):
+    """By rows, by home cells (tricubic) and with the heat deposit; bit-identical to the
+    restatement, whose particles are removed at the same step."""
+    _, cfg, state = make_case(name, seed=8)
+    sets = [k for k in ("p", "g") if k in state]
+    none = (abi.Particle * 0)()
+    ref = O.Restatement(cfg)
+    with ch4b200.Simulation(cfg) as sim:
+        for s in (ref, sim):
+            for k in sets:
+                s.set_pop(k, state[k])
+            s.set_particles(state["part"])
+            s.initialize()
+            s.step(6)
+            s.set_particles(none)
+            s.step(5)
+        for k in sets:
+            assert np.array_equal(sim.get_pop(k), ref.get_pop(k)), k
+    ref.close()

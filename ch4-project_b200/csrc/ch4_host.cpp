@@ -1884,7 +1884,7 @@ struct Engine : EngineBase {
           if (c.resume || n_step > 1) {
             PartParams<A> Q = part_params();
             size_t bytes = cubbytes;
-            if (pslab()) {
+            if (pslab() && mig) {
               // the records of the particles next to a face go to the neighbour, theirs come in
               if (!H->exchange) return H->fail(CH4_ERR_STATE, "z-slab with particles: no ch4_set_exchange");
               const size_t one = MIG_HEAD + (size_t)mig_cap * MIG_REC;
@@ -1958,7 +1958,9 @@ struct Engine : EngineBase {
             rows_ready = Q.emit != 0;
             if ((st = H->cuda(launch_particle_substep(Q, H->stream), "particle substep"))) return st;
             if (rj_random() && np > 0 && (st = reinject_random())) return st;
-            if (pslab() && (st = migrate())) return st;  // move_particles ends with sendrecv_particles
+            // move_particles ends with sendrecv_particles (a lattice without particles has no buffers
+            // for them, on any slab)
+            if (pslab() && mig && (st = migrate())) return st;
           }
         }
       }

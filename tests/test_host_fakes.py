@@ -103,3 +103,33 @@ def test_ensemble_tables_are_ordered_with_the_steps(fakes):
     assert fakes.ch4_ensemble_step(ens, 3) == 0
     assert fakes.fake_faults().decode() == ""
     fakes.ch4_ensemble_destroy(ens)
+
+
+EXCHANGE = C.CFUNCTYPE(C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p, C.c_void_p)
+
+
+@pytest.mark.parametrize("name", ["particles_1w", "particles"])
+@pytest.mark.parametrize("removed", [False, True])
+def test_slab_without_particles(fakes, name, removed):
+    """A slab whose lattice never had particles, or has lost them, has no exchange buffers: it
+    steps without them (and clears its deposit)."""
+    _, cfg, state = make_case(name, seed=1, dims=(6, 5, 8))
+    cfg.nz_global, cfg.z_offset, cfg.NZ = 8, 0, 4
+    state["p"] = state["p"][:4]
+    h = Handle(fakes, cfg, state)
+    moved = EXCHANGE(lambda *a: 0)
+    assert fakes.ch4_set_exchange(h.h, moved, None) == 0 and fakes.ch4_set_face_exchange(h.h, moved, None) == 0
+    if removed:
+        h.set_particles(state["part"])
+    h.initialize()
+    if removed:
+        assert h.step(2) == 0
+        h.set_particles((abi.Particle * 0)())
+    h.log()
+    assert h.step(3) == 0
+    log = h.log()
+    assert log.count("launch_step") == 6  # the face planes, then the interior
+    assert not any("ghosts" in x or "leave" in x or "arrive" in x for x in log)
+    if name == "particles":
+        assert log.count("launch_deposit stage 0") == (3 if removed else 2)
+    h.close()

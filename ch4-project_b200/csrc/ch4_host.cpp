@@ -1331,6 +1331,7 @@ struct Engine : EngineBase {
     a.down = down;
     a.up = up;
     a.pack = pack;
+    if (!(a.word = halo_word(down, up, sbytes))) return H->fail(CH4_ERR_ARG, "face buffers at an odd address");
     const bool local_top[3] = {(F & K_FWALL) && !(F & K_FSLIP_P), (F & K_TWALL) != 0, (F & K_SWALL) != 0};
     const bool local_bot[3] = {(F & K_FWALL) && !(F & K_FSLIP_M), (F & K_TWALL) != 0, (F & K_SWALL) != 0};
     for (int s = 0; s < 3; s++) {

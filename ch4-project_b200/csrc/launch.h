@@ -67,8 +67,17 @@ struct HaloFacesArgs {
   void* pops;
   void* down;
   void* up;
+  size_t word;  // of the accesses to the face buffers: halo_word
   bool pack;
 };
+// the widest word of 2, 4 or 8 bytes, no wider than a stored value, at which both of the caller's
+// face buffers are aligned (0: an odd address).  A library's own buffers give whole values; a
+// buffer inside a packed message may not.
+inline size_t halo_word(const void* down, const void* up, size_t bytes) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(down) | reinterpret_cast<uintptr_t>(up);
+  while (bytes > 1 && at % bytes) bytes /= 2;
+  return bytes > 1 ? bytes : 0;
+}
 cudaError_t launch_halo_faces(const HaloFacesArgs& a, size_t bytes, cudaStream_t st);
 // copies of up to 30 device regions (the u faces of a z-slab), in 4-byte words when every
 // region's size and addresses allow it, else in 2-byte words

@@ -37,7 +37,11 @@ cudaError_t launch_halo_copy(const HaloCopy& H, cudaStream_t st) {
 }
 
 cudaError_t launch_halo_faces(const HaloFacesArgs& a, size_t bytes, cudaStream_t st) {
-  return bytes == 8 ? halo_faces_t<uint64_t>(a, st) : bytes == 4 ? halo_faces_t<uint32_t>(a, st) : halo_faces_t<uint16_t>(a, st);
+  if (a.word == 8) return halo_faces_t<uint64_t, uint64_t>(a, st);
+  if (a.word == 4) return bytes == 8 ? halo_faces_t<uint64_t, uint32_t>(a, st) : halo_faces_t<uint32_t, uint32_t>(a, st);
+  return bytes == 8   ? halo_faces_t<uint64_t, uint16_t>(a, st)
+         : bytes == 4 ? halo_faces_t<uint32_t, uint16_t>(a, st)
+                      : halo_faces_t<uint16_t, uint16_t>(a, st);
 }
 
 cudaError_t launch_step(const StepParams<double>& P, LaunchShape s, cudaStream_t st) {

@@ -603,13 +603,14 @@ __global__ void soa_to_aos_kernel(const S* soa, A* aos, int NX, int NY, int z0, 
 // after the other in a block) and the face buffers: direction k of the five with c_z = -1 (top
 // plane, buffer `down`) or +1 (bottom plane, buffer `up`), planes of NX * NY values by set and
 // direction.  Rows whose values the cell's own wall rule writes stay out (own: bit set for a
-// wall above, bit 3 + set for one below).  PACK: populations -> buffers.
+// wall above, bit 3 + set for one below).  PACK: populations -> buffers.  The caller's buffers are
+// accessed in words W, narrower than a value S where they are not aligned to it.
 struct HaloFaces {
   int NX, NY, NZ, sets;
   uint32_t bstride, own;
 };
-template <typename S, bool PACK>
-__global__ void halo_faces_kernel(S* pops, const HaloFaces H, S* down, S* up) {
+template <typename S, typename W, bool PACK>
+__global__ void halo_faces_kernel(S* pops, const HaloFaces H, W* down, W* up) {
   const long long plane = (long long)H.NX * H.NY, t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= plane) return;
   const int s = blockIdx.y / 10, d = blockIdx.y % 10, y = (int)(t / H.NX);
@@ -618,9 +619,16 @@ __global__ void halo_faces_kernel(S* pops, const HaloFaces H, S* down, S* up) {
     if (cz(q) == (d < 5 ? -1 : 1) && k-- == 0) break;
   if ((cy(q) < 0 && y == H.NY - 1 && ((H.own >> s) & 1)) || (cy(q) > 0 && y == 0 && ((H.own >> (3 + s)) & 1))) return;
   S* cell = pop_at<S>(pops, H.bstride, (d < 5 ? (H.NZ - 1) * plane : 0) + t) + (s * Q + q) * POP_BLOCK;
-  S* face = (d < 5 ? down : up) + ((long long)s * 5 + d % 5) * plane + t;
-  if constexpr (PACK) *face = *cell;
-  else *cell = *face;
+  constexpr int words = sizeof(S) / sizeof(W);
+  W* face = (d < 5 ? down : up) + (((long long)s * 5 + d % 5) * plane + t) * words;
+  // the lowest word first, as the value lies in memory
+  S v = PACK ? *cell : S(0);
+#pragma unroll
+  for (int k = 0; k < words; k++) {
+    if constexpr (PACK) face[k] = (W)(v >> (8 * sizeof(W) * k));
+    else v = (S)(v | ((S)face[k] << (8 * sizeof(W) * k)));
+  }
+  if constexpr (!PACK) *cell = v;
 }
 
 #include "force_moments.cuh"

@@ -407,7 +407,8 @@ ch4_status ch4_halo_bytes(ch4_handle *h, size_t *bytes);
  * the top plane and what the slab below sent up into the bottom plane.  Both run on the
  * handle's stream (the caller's transfer between them must be ordered on it, e.g. NCCL
  * on that stream).  With one slab, from_up = send_down and from_down = send_up give the
- * periodic lattice back. */
+ * periodic lattice back.  The buffers may start at any even address (fastest where aligned
+ * to a stored value; an odd one is refused, CH4_ERR_ARG). */
 ch4_status ch4_halo_pack(ch4_handle *h, void *send_down, void *send_up);
 ch4_status ch4_halo_unpack(ch4_handle *h, const void *from_up, const void *from_down);
 

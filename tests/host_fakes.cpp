@@ -165,7 +165,10 @@ using S = cudaStream_t;
   }
 BOTH(FAKES)
 
-cudaError_t launch_halo_faces(const HaloFacesArgs&, size_t, S st) { return launched("launch_halo_faces", st); }
+cudaError_t launch_halo_faces(const HaloFacesArgs& a, size_t bytes, S st) {
+  if (a.word < 2 || a.word > bytes || ((size_t)a.down | (size_t)a.up) % a.word) g_faults += "launch_halo_faces: word\n";
+  return launched("launch_halo_faces", st, "word " + std::to_string(a.word));
+}
 cudaError_t launch_halo_copy(const HaloCopy&, S st) { return launched("launch_halo_copy", st); }
 cudaError_t launch_particle_records(const double*, int, int, int, double*, S st) { return launched("launch_particle_records", st); }
 cudaError_t launch_particle_averages(const double*, int, int, double*, int, double*, S st) {

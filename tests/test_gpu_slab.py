@@ -5,6 +5,8 @@ FP32: every cell does the same arithmetic; HIT tables run over the whole lattice
 The slabs of one process unpack straight from their neighbours' send buffers; the
 multi-rank exchange over torch.distributed is covered on CPU (tests/test_slab_exchange.py).
 """
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -276,3 +278,37 @@ def test_particles_on_slabs_refuse_walls_and_the_folded_deposits():
         _, cfg, _ = make_case(name, seed=48)
         with pytest.raises(ch4b200.CH4Error):
             slab.Slab(cfg, 0, cfg.NZ // 2)
+
+
+@pytest.mark.parametrize("storage,at", [(0, 4), (0, 2), (1, 2), (2, 2)])
+def test_faces_in_buffers_of_narrow_alignment(storage, at):
+    """Packed into and unpacked from buffers `at` bytes past an aligned address, the faces are
+    those of aligned buffers (the wall rows of the Rayleigh-Benard case stay out), and the bytes
+    around them are untouched."""
+    _, cfg, state = make_case("rb", seed=3, storage=storage)
+    with ch4b200.Simulation(cfg) as sim:
+        L, n = ch4b200.lib(), C.c_size_t()
+        assert L.ch4_halo_bytes(sim.h, C.byref(n)) == 0
+        n = n.value
+
+        def faces(off):
+            bufs = [torch.full((n + 32,), 7, dtype=torch.uint8, device="cuda") for _ in range(2)]
+            torch.cuda.synchronize()
+            ptr = [b.data_ptr() + off for b in bufs]
+            assert all(b.data_ptr() % 256 == 0 for b in bufs)
+            for k, v in pop_items(state):
+                sim.set_pop(k, v)
+            assert L.ch4_halo_pack(sim.h, *ptr) == 0
+            sim.synchronize()
+            out = [b.clone() for b in bufs]
+            for k, v in pop_items(state):  # other populations: the faces come from the buffers alone
+                sim.set_pop(k, 2.0 * v)
+            assert L.ch4_halo_unpack(sim.h, *ptr) == 0
+            sim.synchronize()
+            return out, [sim.get_pop(k) for k, _ in pop_items(state)]
+
+        (a, pa), (b, pb) = faces(0), faces(at)
+        for x, y in zip(a, b):
+            assert torch.equal(x[:n], y[at:at + n])
+            assert (y[:at] == 7).all() and (y[at + n:] == 7).all()
+        assert all(np.array_equal(x, y) for x, y in zip(pa, pb))

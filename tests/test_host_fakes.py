@@ -133,3 +133,18 @@ def test_slab_without_particles(fakes, name, removed):
     if name == "particles":
         assert log.count("launch_deposit stage 0") == (3 if removed else 2)
     h.close()
+
+
+@pytest.mark.parametrize("storage,at,word", [(0, (0, 0), 8), (0, (4, 0), 4), (0, (0, 12), 4), (0, (8, 2), 2), (1, (4, 8), 4),
+                                             (1, (0, 6), 2), (2, (2, 0), 2), (0, (1, 0), None), (2, (0, 3), None)])
+def test_face_buffers_of_any_alignment(fakes, storage, at, word):
+    """Face buffers aligned to less than a stored value go through narrower words; an odd
+    address is refused."""
+    _, cfg, state = make_case("rb", seed=1, storage=storage)
+    h = Handle(fakes, cfg, state)
+    h.log()
+    down, up = (C.c_void_p((1 << 20) + a) for a in at)
+    for call in (fakes.ch4_halo_pack, fakes.ch4_halo_unpack):
+        assert call(h.h, down, up) == (abi.ERR_ARG if word is None else abi.OK)
+        assert h.log() == ([] if word is None else ["launch_halo_faces word %d" % word])
+    h.close()

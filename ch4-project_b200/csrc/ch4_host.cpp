@@ -1075,16 +1075,20 @@ struct Engine : EngineBase {
     }
   }
 
+  // no place of the row lists is drawn: the next deposit draws them from the state
+  ch4_status clear_rows() {
+    rows_ready = false;
+    if (!row_count) return CH4_OK;
+    const size_t nb = row_bins(c.NX, c.NY, c.NZ);
+    return H->cuda(cudaMemsetAsync(row_count, 0, sizeof(int) * (nb + 1), H->stream), "row lists");
+  }
+
   ch4_status set_particles(const ch4_particle* parts, int n) override {
     if (!lagr()) return H->fail(CH4_ERR_ARG, "particles need the LAGRANGE flag");
     if (n < 0 || (n > 0 && !parts)) return H->fail(CH4_ERR_ARG, "bad particle array");
     ch4_status st;
     if ((st = H->cuda(cudaStreamSynchronize(H->stream), "sync"))) return st;
-    if (rows_ready) {  // places drawn for a deposit that will not come
-      const size_t nb = row_bins(c.NX, c.NY, c.NZ);
-      if ((st = H->cuda(cudaMemsetAsync(row_count, 0, sizeof(int) * (nb + 1), H->stream), "row lists"))) return st;
-    }
-    rows_ready = false;
+    if ((st = clear_rows())) return st;  // places drawn for a deposit that will not come
     const bool sl = pslab();
     if (n != (sl ? np_all : np) || (sl && !mig)) {
       free_particles();
@@ -1901,7 +1905,11 @@ struct Engine : EngineBase {
               // (the sort holds ghosts too: the slots are re-sorted on their own)
               if (np > 0 && ++since_reorder >= REORDER_EVERY && (st = reorder_particles(1))) return st;
             } else {
-              if ((st = H->cuda(launch_deposit(Q, key2, order2, cubtmp, bytes, H->stream), "deposit"))) return st;
+              if ((st = H->cuda(launch_deposit(Q, key2, order2, cubtmp, bytes, H->stream), "deposit"))) {
+                clear_rows();
+                return st;
+              }
+              rows_ready = false;  // used up: a step that fails from here on is followed by a deposit from the state
               // (unless by rows, the deposit's sort already holds the slots in home-cell order)
               if (np > 0 && ++since_reorder >= REORDER_EVERY && (st = reorder_particles(by_rows() ? 1 : 0))) return st;
             }
@@ -1939,6 +1947,7 @@ struct Engine : EngineBase {
         }
         if (fmoments()) fm_i ^= 1;
         cur ^= 1;
+        upart_current = false;
         H->itime++;
         H->time_now += c.time_dt;
         if (lagr()) {
@@ -1956,8 +1965,8 @@ struct Engine : EngineBase {
             Q.first = (n_step == 1 && c.resume == 0);
             Q.time_now = H->time_now;
             Q.emit = by_rows() && !rj_random() && sub + 1 == (int)c.time_dt_lagr_factor;
-            rows_ready = Q.emit != 0;
             if ((st = H->cuda(launch_particle_substep(Q, H->stream), "particle substep"))) return st;
+            rows_ready = Q.emit != 0;
             if (rj_random() && np > 0 && (st = reinject_random())) return st;
             // move_particles ends with sendrecv_particles (a lattice without particles has no buffers
             // for them, on any slab)

@@ -1,7 +1,7 @@
 // The CUDA runtime and the kernel launchers, faked on the host, so that the library's host code
 // (csrc/ch4_host.cpp) runs without a GPU: device memory is host memory, copies and clears happen
 // at once, launchers do nothing.  What a test asks about is written down:
-//   fake_log()     one line per launch
+//   fake_log()     one line per launch or clear
 //   fake_faults()  one line per call whose result a GPU would not promise
 //   fake_fail(f)   the next call of f returns an error
 //
@@ -57,6 +57,7 @@ cudaError_t cudaMemset(void* p, int v, size_t n) {
 }
 cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t st) {
   std::memset(p, v, n);
+  g_log += "clear " + std::to_string(n) + "\n";
   return ordered("cudaMemsetAsync", st);
 }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind k) {

@@ -148,3 +148,41 @@ def test_face_buffers_of_any_alignment(fakes, storage, at, word):
         assert call(h.h, down, up) == (abi.ERR_ARG if word is None else abi.OK)
         assert h.log() == ([] if word is None else ["launch_halo_faces word %d" % word])
     h.close()
+
+
+@pytest.mark.parametrize("failing", ["launch_step", "launch_hydro", "launch_deposit", "launch_particle_substep"])
+def test_deposit_after_a_failed_step_takes_the_state(handle, fakes, failing):
+    """The lists that the last sub-step began serve one deposit.  A step that fails after it, or
+    in it, is followed by a deposit that lists the particles itself, from cleared counters."""
+    h, state = handle("particles")
+    h.set_particles(state["part"])
+    h.initialize()
+    assert h.step(3) == 0
+    assert h.log().count("launch_deposit stage 0 ready") == 2
+    fakes.fake_fail(failing.encode())
+    assert h.step() != 0
+    bins = (h.cfg.NY + 1) * (h.cfg.NZ + 1)
+    failed = h.log()
+    assert ("clear %d" % (4 * (bins + 1)) in failed) == (failing == "launch_deposit")
+    assert h.step() == 0
+    assert [x for x in h.log() if "deposit" in x] == ["launch_deposit stage 0"]
+    assert h.step() == 0
+    assert "launch_deposit stage 0 ready" in h.log()
+
+
+def test_u_of_the_les_after_a_failed_step(handle, fakes):
+    """With particles the LES takes u^n from the vectors the last step formed for them; where
+    that step failed before it formed them, u^n is computed."""
+    h, state = handle("particles_1w")
+    h.cfg.flags |= abi.FLAGS["LB_FLUID_LES"]
+    les = Handle(fakes, h.cfg, {"p": state["p"]})
+    les.initialize()
+    les.log()
+    counts = []
+    for fail in (False, False, True, False, False):
+        if fail:
+            fakes.fake_fail(b"launch_hydro")
+        assert (les.step() != 0) == fail
+        counts.append(les.log().count("launch_hydro"))
+    assert counts == [2, 1, 1, 2, 1]
+    les.close()

@@ -912,6 +912,7 @@ struct Engine : EngineBase {
                                                                                     : 1;
     Q.nrec = nrec();
     Q.rows = by_rows();
+    Q.segs = row_segs(c.NX);
     Q.rows_ready = rows_ready;
     Q.row_place = row_place;
     Q.row_count = row_count;
@@ -1079,7 +1080,7 @@ struct Engine : EngineBase {
   ch4_status clear_rows() {
     rows_ready = false;
     if (!row_count) return CH4_OK;
-    const size_t nb = row_bins(c.NX, c.NY, c.NZ);
+    const size_t nb = row_bins(row_segs(c.NX), c.NY, c.NZ);
     return H->cuda(cudaMemsetAsync(row_count, 0, sizeof(int) * (nb + 1), H->stream), "row lists");
   }
 
@@ -1104,8 +1105,8 @@ struct Engine : EngineBase {
                     cudaMalloc(&order, sizeof(int) * n) == cudaSuccess &&
                     cudaMalloc(&order2, sizeof(int) * n) == cudaSuccess &&
                     (!twoway() || cudaMalloc(&rec, sizeof(double) * nrec() * (size_t)n) == cudaSuccess) &&
-                    (!by_rows() || (cudaMalloc(&row_place, sizeof(int2) * (size_t)n) == cudaSuccess &&
-                                    cudaMalloc(&row_entry, sizeof(int2) * (size_t)n) == cudaSuccess)) &&
+                    (!by_rows() || (cudaMalloc(&row_place, sizeof(int2) * row_places(row_segs(c.NX)) * (size_t)n) == cudaSuccess &&
+                                    cudaMalloc(&row_entry, sizeof(int2) * row_places(row_segs(c.NX)) * (size_t)n) == cudaSuccess)) &&
                     (!twoway() || by_rows() || (cudaMalloc(&srec, sizeof(double) * nrec() * (size_t)n) == cudaSuccess &&
                                                 cudaMalloc(&spid, sizeof(int) * (size_t)n) == cudaSuccess));
           if (!ok) return H->fail(CH4_ERR_NOMEM, "sort buffers");
@@ -1459,7 +1460,7 @@ struct Engine : EngineBase {
       }
       const size_t nreg = (size_t)((c.NX + GATHER_BLOCK - 1) / GATHER_BLOCK) * c.NY * c.NZ;
       if (by_rows()) {
-        const size_t nb = row_bins(c.NX, c.NY, c.NZ);
+        const size_t nb = row_bins(row_segs(c.NX), c.NY, c.NZ);
         if (cudaMalloc(&row_count, sizeof(int) * (nb + 1)) != cudaSuccess ||
             cudaMalloc(&row_list, sizeof(int2) * nb) != cudaSuccess)
           return H->fail(CH4_ERR_NOMEM, "row lists");

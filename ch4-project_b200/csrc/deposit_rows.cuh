@@ -13,6 +13,14 @@
 // the particles fills them in, and a last one puts every list in particle-index order -- the
 // order of the draws is the schedule's, the lists and sums are not.
 //
+// Rows longer than ROW_SEG are cut into segments of ROW_CUT cells.  A segment's last cell also takes
+// from the next segment's first home cell; the particles of that home are listed a second time, in
+// an edge list of their own, so that no warp reads the next segment's whole list for them.  us a step
+// FP32, by home cells / rows with the next segment's list merged whole / with edge lists and 256
+// cells a segment / 128: 512x128x64 with 0.06 particles a cell 442 / 495 / 404 / 384, with 0.25 776 /
+// 1,265 / 829 / 720, with 0.008 351 / 290 / 288 / 294; 300x128x96 (256 + 44 cells left half of the
+// warps with most of the work) with 0.11 476 / 605 / 499 / 412.
+//
 // Why rows: at the workloads' 0.04 depositing particles per cell nearly every home cell is
 // empty, and a list per home cell (a range of 8 bytes each, cleared, filled, read and scanned
 // every step) moved more bytes than the particles; a row of 256 cells has some 10 particles a
@@ -22,20 +30,39 @@
 // 1,155 -> 1,073 (four launches of the sort and the copy of the records into its order gone).
 #pragma once
 
-constexpr int ROW_SEG = 256;    // cells of a row that one warp owns
-constexpr int ROW_CHUNK = 64;   // merged entries in shared memory at a time (8 lists x 8)
+constexpr int ROW_SEG = 256;    // cells of a row that one warp owns, at most
+constexpr int ROW_CUT_SHIFT = 7, ROW_CUT = 1 << ROW_CUT_SHIFT;  // cells of a segment of a longer row
+constexpr int ROW_CHUNK = 64;   // merged entries in shared memory at a time
 constexpr int ROW_WARPS = 4;    // warps per block
 constexpr int ROW_REC = 10;     // doubles of a record: fac*fp (3), dxm dxp dym dyp dzm dzp, {hx, index}
 
-// row segments along x: the last home cell (hx = NX) belongs to the last segment
-__host__ __device__ __forceinline__ int row_segs(int NX) { return (NX + ROW_SEG - 1) / ROW_SEG; }
-__host__ __device__ __forceinline__ unsigned int row_bins(int NX, int NY, int NZ) {
-  return (unsigned)row_segs(NX) * (unsigned)(NY + 1) * (unsigned)(NZ + 1);
+// the segments of a row of NX cells: all of `len` cells but for the last; the last home cell (hx =
+// NX) belongs to the last segment
+inline RowSegs row_segs(int NX) {
+  if (NX <= ROW_SEG) return {1, NX, 31};
+  return {(NX + ROW_CUT - 1) / ROW_CUT, ROW_CUT, ROW_CUT_SHIFT};
 }
-__host__ __device__ __forceinline__ unsigned int row_bin(int hx, int hy, int hz, int NX, int NY) {
-  const int ns = row_segs(NX), s = hx / ROW_SEG;
-  return ((unsigned)hz * (unsigned)(NY + 1) + (unsigned)hy) * (unsigned)ns + (unsigned)(s < ns ? s : ns - 1);
+// lists of one home row: its segments', then the edge lists of the first home cells of segments
+// 1 .. (home len s is the first of segment s)
+__host__ __device__ __forceinline__ unsigned int row_lists(const RowSegs& g) { return 2u * (unsigned)g.n - 1u; }
+inline unsigned int row_bins(const RowSegs& g, int NY, int NZ) {
+  return row_lists(g) * (unsigned)(NY + 1) * (unsigned)(NZ + 1);
 }
+__host__ __device__ __forceinline__ int row_seg(int hx, const RowSegs& g) {
+  const int s = hx >> g.shift;
+  return s < g.n ? s : g.n - 1;
+}
+// the list of a home cell, and its edge list or -1
+__host__ __device__ __forceinline__ int row_bin(int hx, int hy, int hz, const RowSegs& g, int NY) {
+  return (int)(((unsigned)hz * (unsigned)(NY + 1) + (unsigned)hy) * row_lists(g)) + row_seg(hx, g);
+}
+__host__ __device__ __forceinline__ int row_edge_bin(int hx, int hy, int hz, const RowSegs& g, int NY) {
+  const int s = row_seg(hx, g);
+  if (s == 0 || hx != s * g.len) return -1;
+  return (int)(((unsigned)hz * (unsigned)(NY + 1) + (unsigned)hy) * row_lists(g)) + g.n + s - 1;
+}
+// places of a particle: one, and with edge lists a second
+__host__ __device__ __forceinline__ int row_places(const RowSegs& g) { return g.n > 1 ? 2 : 1; }
 
 #ifdef __CUDACC__
 
@@ -56,11 +83,15 @@ __device__ __forceinline__ void deposit_rows_emit(const PartParams<A>& P, int ip
   const int o = P.pid[ip];
   const bool live = inside && (fac > 0.0) && beta != 0.0;
   const int hx = t.im + 1, hy = t.jm + 1, hz = t.km + 1;
+  if (P.segs.n > 1) {
+    const int edge = live ? row_edge_bin(hx, hy, hz, P.segs, P.NY) : -1;
+    P.row_place[np + ip] = make_int2(edge, edge < 0 ? 0 : atomicAdd(P.row_count + edge, 1));
+  }
   if (!live) {
     P.row_place[ip] = make_int2(-1, 0);
     return;
   }
-  const int bin = (int)row_bin(hx, hy, hz, P.NX, P.NY);
+  const int bin = row_bin(hx, hy, hz, P.segs, P.NY);
   P.row_place[ip] = make_int2(bin, atomicAdd(P.row_count + bin, 1));
   const double dr = pf[PF_DR * np + ip];
   double aa[3], DD[3];
@@ -122,14 +153,16 @@ static __global__ void row_ranges_kernel(int* count, unsigned int nb, int2* list
 }
 
 // the particles into their lists, as {index, slot}
-static __global__ void row_fill_kernel(const int2* place, const int2* list, const int* pid, int np, int2* entry,
-                                       int* cursor) {
+static __global__ void row_fill_kernel(const int2* place, int places, const int2* list, const int* pid, int np,
+                                       int2* entry, int* cursor) {
   grid_chain();
   const int ip = blockIdx.x * blockDim.x + threadIdx.x;
   if (ip == 0) *cursor = 0;  // for the next deposit
   if (ip >= np) return;
-  const int2 p = place[ip];
-  if (p.x >= 0) entry[list[p.x].x + p.y] = make_int2(pid[ip], ip);
+  for (int k = 0; k < places; k++) {
+    const int2 p = place[(long long)k * np + ip];
+    if (p.x >= 0) entry[list[p.x].x + p.y] = make_int2(pid[ip], ip);
+  }
 }
 
 // every list in particle-index order, a warp per list: up to 32 entries ranked in registers, more
@@ -167,9 +200,9 @@ static __global__ void row_order_kernel(const int2* list, unsigned int nb, int2*
 
 // shared memory of one warp: the contributions by merged position (component c of corner di
 // at 2 c + di), the row's sums (three rows of `cells`), indices and cells of the merged entries
-__host__ __device__ __forceinline__ int row_cells(int NX) { return (NX < ROW_SEG ? NX : ROW_SEG) + 1; }  // and a spare one
-__host__ __device__ __forceinline__ int row_shared(int NX) {
-  return ROW_CHUNK * 6 * 8 + 3 * row_cells(NX) * 8 + ROW_CHUNK * 3 * 4;
+__host__ __device__ __forceinline__ int row_cells(const RowSegs& g) { return g.len + 1; }  // and a spare one
+__host__ __device__ __forceinline__ int row_shared(const RowSegs& g) {
+  return ROW_CHUNK * 6 * 8 + 3 * row_cells(g) * 8 + ROW_CHUNK * 3 * 4;
 }
 
 // what a record of list l adds to the two cells it has in the row of n cells: component c of
@@ -206,27 +239,28 @@ __device__ __forceinline__ void row_accumulate(int merged, int lane, int cells, 
   __syncwarp();
 }
 
-template <typename A>
+// nl: lists of a warp, 4, or 8 where rows are cut
+template <typename A, int nl>
 __global__ void __launch_bounds__(32 * ROW_WARPS) deposit_rows_kernel(const PartParams<A> P) {
   grid_chain();
   extern __shared__ double row_smem[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cells = row_cells(P.NX);
-  double* const con = row_smem + warp * (row_shared(P.NX) / 8);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cells = row_cells(P.segs);
+  double* const con = row_smem + warp * (row_shared(P.segs) / 8);
   double* const acc = con + ROW_CHUNK * 6;
   int* const s_pid = reinterpret_cast<int*>(acc + 3 * cells);
   int* const s_at = s_pid + ROW_CHUNK;
-  const int ns = row_segs(P.NX), nl = ns == 1 ? 4 : 8;  // lists
+  const int ns = nl == 4 ? 1 : P.segs.n;
   const unsigned int w = blockIdx.x * ROW_WARPS + warp;  // of plane k's ns * NY
-  const int j = (int)(ns == 1 ? w : w / (unsigned)ns), seg = (int)w - j * ns, k = blockIdx.y;
+  const int j = (int)(nl == 4 ? w : w / (unsigned)ns), seg = (int)w - j * ns, k = blockIdx.y;
   if (j >= P.NY) return;  // whole warps: no block barrier below
-  const int x0 = seg * ROW_SEG, n = min(ROW_SEG, P.NX - x0);
+  const int x0 = seg * P.segs.len, n = min(P.segs.len, P.NX - x0);
   A* out = P.dep + ((long long)k * P.NY + j) * P.NX + x0;
   // lane l < 4: the home row (y + (l & 1), z + (l >> 1)) of this segment; 4 <= l < 8: the same
-  // rows' next segment, whose first home cell also deposits into this one's last cell
+  // rows' edge list, of the next segment's first home cell
   int beg = 0, end = 0;
-  if (lane < 8 && (lane < 4 || seg + 1 < ns)) {
+  if (lane < nl && (lane < 4 || seg + 1 < ns)) {
     const unsigned int b = ((unsigned)(k + ((lane >> 1) & 1)) * (unsigned)(P.NY + 1) + (unsigned)(j + (lane & 1))) *
-                               (unsigned)ns + (unsigned)(seg + (lane >> 2));
+                               row_lists(P.segs) + (unsigned)(lane < 4 ? seg : ns + seg);
     const int2 range = P.row_list[b];
     beg = range.x;
     end = range.y;
@@ -266,7 +300,8 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) deposit_rows_kernel(const Part
     // up to the smallest index T that ends a cut list are merged now
     while (__any_sync(ALL, beg < end)) {
       const int left = __reduce_add_sync(ALL, end - beg);
-      const int cap = left <= ROW_CHUNK ? ROW_CHUNK : ROW_CHUNK / (ns == 1 ? 4 : 8);
+      // (an edge list holds the particles of one home cell, the others those of a segment's)
+      const int cap = left <= ROW_CHUNK ? ROW_CHUNK : nl == 4 ? ROW_CHUNK / 4 : lane < 4 ? ROW_CHUNK / 4 - 2 : 2;
       const int cnt = min(end - beg, cap);
       int off = cnt;  // inclusive prefix over the lists, then exclusive
 #pragma unroll

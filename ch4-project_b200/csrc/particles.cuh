@@ -50,6 +50,11 @@ struct PartPlanes {
   unsigned char f[PF_TOTAL];
 };
 
+// the segments that the deposit by rows cuts the lattice's rows into (row_segs)
+struct RowSegs {
+  int n, len, shift;
+};
+
 template <typename A>
 struct PartParams {
   int NX, NY, NZ;
@@ -87,12 +92,13 @@ struct PartParams {
   // trilinear momentum deposit by lattice rows (deposit_rows.cuh): rec then holds ROW_REC
   // doubles per state slot, one record after the other
   int rows;
+  RowSegs segs;
   int rows_ready;        // the last sub-step wrote the records and places
   int emit;              // this sub-step writes them
-  int2* row_place;       // [np] by slot: list and place in it (-1: deposits nothing)
+  int2* row_place;       // [row_places][np] by slot: list and place in it (-1: none)
   int* row_count;        // [row_bins] places drawn, then the cursor that the lists' ranges are drawn from
   int2* row_list;        // [row_bins] first entry and end of every list
-  int2* row_entry;       // [np] {index, slot} by list
+  int2* row_entry;       // [row_places * np] {index, slot} by list
   double* srec;          // [nrec][np] the same by sorted position (depositing particles only)
   int* spid;             // particle index by sorted position
   int2* cell_rng;        // [(NX+1)(NY+1)(NZ+1)] {start, end} of every home cell's sorted run

@@ -63,6 +63,24 @@ def test_rows_bit_identical(name):
         assert np.array_equal(got[k], v), k
 
 
+@pytest.mark.parametrize("nx,ends", [(257, (128, 256)), (300, (128, 256)), (512, (128, 256, 384)), (515, (128, 384, 512))])
+@pytest.mark.parametrize("n,steps", [(150, 6), (900, 3)])
+def test_cut_rows(nx, ends, n, steps):
+    """Rows of three to five segments, a third of the particles about the segments' ends: in the
+    lists of the segment and in the edge lists of the one before; up to and beyond the 32 and the
+    64 entries that a warp takes at once."""
+    dims = (nx, 4, 3)
+    _, cfg, state = make_case("particles", seed=2, dims=dims)
+    at = tuple(e + d for e in ends for d in (0.0, 0.5, 1.0))
+    parts = small_particles(np.random.default_rng(nx), n, dims, (nx, 2, 2), at)
+    ref = run_restatement(cfg, dict(state, part=parts), steps)
+    assert np.isfinite(ref["p"]).all()
+    p, got = run(cfg, state, parts, steps)
+    assert np.array_equal(p, ref["p"])
+    for k, v in ref["part"].items():
+        assert np.array_equal(got[k], v), k
+
+
 @pytest.mark.parametrize("name", ["segments", "dense"])
 def test_rows_f32_reproducible(name):
     c = CASES[name]

@@ -728,6 +728,16 @@ struct Engine : EngineBase {
   int* row_count = nullptr;
   int2* row_list = nullptr;
   int2 *row_place = nullptr, *row_entry = nullptr;
+  // The deposit goes by rows while the lists are short (row_limit), else by home cells.  The longest
+  // list is watched on the device; its figure is asked for at every LOOK_EVERY-th re-sort and used at
+  // the next, 256 steps later: the choice does not depend on timing, and the host, which is ahead by
+  // no more launches than the queue holds, does not wait for it.
+  static constexpr int LOOK_EVERY = 16;
+  int sorts_done = 0;
+  bool rows_on = true;
+  int *row_longest = nullptr, *row_longest_h = nullptr;
+  cudaEvent_t row_ev = nullptr;
+  bool row_asked = false;   // row_longest_h is on its way or there
   bool rows_ready = false;  // its records and places are those of the state (the last sub-step wrote them)
   int2* crng = nullptr;   // {start, end} per home cell
   int* busy = nullptr;    // cells for the deposit merge pass, per gather block
@@ -787,13 +797,12 @@ struct Engine : EngineBase {
     cudaFree(upart);
     cudaFree(dbuf[0]);
     cudaFree(dbuf[1]);
-    cudaFree(crng);
     cudaFree(row_count);
     cudaFree(row_list);
-    cudaFree(busy);
-    cudaFree(bcount);
-    cudaFree(boff);
-    cudaFree(dense);
+    cudaFree(row_longest);
+    cudaFreeHost(row_longest_h);
+    if (row_ev) cudaEventDestroy(row_ev);
+    free_home();
     cudaFree(pstatus);
     cudaFree(fmbuf);
     cudaFree(fmpart);
@@ -845,12 +854,13 @@ struct Engine : EngineBase {
 
   size_t nhome() const { return (size_t)(c.NX + 1) * (c.NY + 1) * (c.NZ + 1); }
   bool twoway_temp() const { return (c.flags2 & CH4_F2_LAGRANGE_TWOWAY_TEMPERATURE) != 0; }
-  // deposit record fields: fac*fp (3) + the stencil weights (6 trilinear, 12 tricubic), then
-  // with the thermal coupling fac*sp
-  // the plain trilinear momentum deposit of a whole lattice goes by rows (deposit_rows.cuh)
-  bool by_rows() const {
+  // the plain trilinear momentum deposit of a whole lattice can go by rows (deposit_rows.cuh)
+  bool rows_able() const {
     return twoway() && !twoway_temp() && !pslab() && !(c.flags & CH4_F_LAGRANGE_TWOWAY_TRICUBIC);
   }
+  bool by_rows() const { return rows_able() && rows_on; }
+  // deposit record fields: fac*fp (3) + the stencil weights (6 trilinear, 12 tricubic), then
+  // with the thermal coupling fac*sp
   int nrec() const { return by_rows() ? ROW_REC : ((c.flags & CH4_F_LAGRANGE_TWOWAY_TRICUBIC) ? 15 : 9) + (twoway_temp() ? 1 : 0); }
   // planes of a deposit buffer: the force, and the temperature source with the thermal coupling
   int dplanes() const { return twoway_temp() ? 4 : 3; }
@@ -918,6 +928,7 @@ struct Engine : EngineBase {
     Q.row_count = row_count;
     Q.row_list = row_list;
     Q.row_entry = row_entry;
+    Q.row_longest = row_longest;
     Q.rec = rec;
     Q.srec = srec;
     Q.spid = spid;
@@ -1076,6 +1087,75 @@ struct Engine : EngineBase {
     }
   }
 
+  // the buffers of the deposit by home cells: of the lattice, and of n particles
+  bool home_buffers() {
+    const size_t nreg = (size_t)((c.NX + GATHER_BLOCK - 1) / GATHER_BLOCK) * c.NY * c.NZ;
+    return boff || (cudaMalloc(&crng, sizeof(int2) * nhome()) == cudaSuccess &&
+                    cudaMalloc(&busy, sizeof(int) * nreg * GATHER_BLOCK) == cudaSuccess &&
+                    cudaMalloc(&dense, sizeof(int) * nreg * GATHER_BLOCK) == cudaSuccess &&
+                    cudaMalloc(&bcount, sizeof(int) * nreg) == cudaSuccess &&
+                    cudaMalloc(&boff, sizeof(int) * nreg) == cudaSuccess);
+  }
+  void free_home() {
+    for (void* b : {(void*)crng, (void*)busy, (void*)dense, (void*)bcount, (void*)boff}) cudaFree(b);
+    crng = nullptr;
+    busy = dense = bcount = boff = nullptr;
+  }
+  bool sorted_buffers(int n) {
+    const size_t fields = (c.flags & CH4_F_LAGRANGE_TWOWAY_TRICUBIC ? 15 : 9) + (twoway_temp() ? 1 : 0);
+    return spid || (cudaMalloc(&srec, sizeof(double) * fields * (size_t)n) == cudaSuccess &&
+                    cudaMalloc(&spid, sizeof(int) * (size_t)n) == cudaSuccess);
+  }
+
+  // The route of the next deposit.  Both add every cell's particles in index order (FP64: the same
+  // bits; FP32 contracts the products of one of them).  Without the memory for home cells it stays by rows.
+  ch4_status go_by_rows(bool rows) {
+    if (!rows && !(home_buffers() && sorted_buffers(np))) {
+      cudaGetLastError();  // the refused allocation
+      if (!boff) free_home();
+      if (!spid) {
+        cudaFree(srec);
+        srec = nullptr;
+      }
+      rows = true;
+    }
+    if (rows == rows_on) return CH4_OK;
+    rows_on = rows;
+    return clear_rows();
+  }
+
+  // the longest list that the deposit by rows would have (the positions are finite)
+  int longest_row(const std::vector<double>& h, size_t n) const {
+    const RowSegs g = row_segs(c.NX);
+    std::vector<int> count(row_bins(g, c.NY, c.NZ), 0);
+    const double *x = &h[(size_t)CH4_PF(x) * n], *y = &h[(size_t)CH4_PF(y) * n], *z = &h[(size_t)CH4_PF(z) * n];
+    const double *vol = &h[(size_t)PF_VOL * n], *beta = &h[(size_t)CH4_PF(beta_coeff) * n];
+    auto home = [](double v, double S, int m) { return std::min(std::max((int)std::floor(pwrapd(v, S) - 0.5) + 1, 0), m); };
+    int most = 0;
+    for (size_t i = 0; i < n; i++)
+      if (vol[i] > 0.0 && beta[i] != 0.0)
+        most = std::max(most, ++count[row_bin(home(x[i], c.SX, c.NX), home(y[i], c.SY, c.NY), home(z[i], c.SZ, c.NZ), g,
+                                              c.NY)]);
+    return most;
+  }
+
+  // the route by the figure asked for at the last look
+  ch4_status choose_route() {
+    if (!row_asked) return CH4_OK;
+    row_asked = false;
+    if (ch4_status st = H->cuda(cudaEventSynchronize(row_ev), "row lists")) return st;
+    return go_by_rows(*row_longest_h <= (rows_on ? row_limit(row_segs(c.NX)) : row_resume(row_segs(c.NX))));
+  }
+  ch4_status ask_longest() {
+    ch4_status st;
+    if ((st = H->cuda(cudaMemcpyAsync(row_longest_h, row_longest, sizeof(int), cudaMemcpyDeviceToHost, H->stream), "row lists")) ||
+        (st = H->cuda(cudaMemsetAsync(row_longest, 0, sizeof(int), H->stream), "row lists")) ||
+        (st = H->cuda(cudaEventRecord(row_ev, H->stream), "row lists")))
+      return st;
+    row_asked = true;
+    return CH4_OK;
+  }
+
   // no place of the row lists is drawn: the next deposit draws them from the state
   ch4_status clear_rows() {
     rows_ready = false;
@@ -1104,11 +1184,10 @@ struct Engine : EngineBase {
                     cudaMalloc(&key2, sizeof(unsigned) * n) == cudaSuccess &&
                     cudaMalloc(&order, sizeof(int) * n) == cudaSuccess &&
                     cudaMalloc(&order2, sizeof(int) * n) == cudaSuccess &&
-                    (!twoway() || cudaMalloc(&rec, sizeof(double) * nrec() * (size_t)n) == cudaSuccess) &&
-                    (!by_rows() || (cudaMalloc(&row_place, sizeof(int2) * row_places(row_segs(c.NX)) * (size_t)n) == cudaSuccess &&
-                                    cudaMalloc(&row_entry, sizeof(int2) * row_places(row_segs(c.NX)) * (size_t)n) == cudaSuccess)) &&
-                    (!twoway() || by_rows() || (cudaMalloc(&srec, sizeof(double) * nrec() * (size_t)n) == cudaSuccess &&
-                                                cudaMalloc(&spid, sizeof(int) * (size_t)n) == cudaSuccess));
+                    (!twoway() || cudaMalloc(&rec, sizeof(double) * (rows_able() ? ROW_REC : nrec()) * (size_t)n) == cudaSuccess) &&
+                    (!rows_able() || (cudaMalloc(&row_place, sizeof(int2) * row_places(row_segs(c.NX)) * (size_t)n) == cudaSuccess &&
+                                      cudaMalloc(&row_entry, sizeof(int2) * row_places(row_segs(c.NX)) * (size_t)n) == cudaSuccess)) &&
+                    (!twoway() || rows_able() || sorted_buffers(n));
           if (!ok) return H->fail(CH4_ERR_NOMEM, "sort buffers");
           if (rj_random() && (cudaMalloc(&rj_count, sizeof(int) * (size_t)n) != cudaSuccess ||
                               cudaMalloc(&rj_xz, 2 * sizeof(double) * (size_t)n) != cudaSuccess))
@@ -1176,6 +1255,13 @@ struct Engine : EngineBase {
                        "particles up"))))
       return st;
     find_planes(h, n);
+    if (rows_able()) {
+      row_asked = false;
+      sorts_done = 0;
+      if ((st = H->cuda(cudaMemsetAsync(row_longest, 0, sizeof(int), H->stream), "row lists")) ||
+          (st = go_by_rows(longest_row(h, n) <= row_limit(row_segs(c.NX)))))
+        return st;
+    }
     since_reorder = REORDER_EVERY;  // sort at the first opportunity
     if (n == 0) return CH4_OK;
     return upload(pid, ids.data(), sizeof(int) * n, "particle ids up");
@@ -1458,19 +1544,19 @@ struct Engine : EngineBase {
         if (cudaMemsetAsync(dbuf[b], 0, dplanes() * N * sizeof(A), H->stream) != cudaSuccess)
           return H->fail(CH4_ERR_CUDA, "deposit memset");
       }
-      const size_t nreg = (size_t)((c.NX + GATHER_BLOCK - 1) / GATHER_BLOCK) * c.NY * c.NZ;
-      if (by_rows()) {
+      if (rows_able()) {
         const size_t nb = row_bins(row_segs(c.NX), c.NY, c.NZ);
         if (cudaMalloc(&row_count, sizeof(int) * (nb + 1)) != cudaSuccess ||
-            cudaMalloc(&row_list, sizeof(int2) * nb) != cudaSuccess)
+            cudaMalloc(&row_list, sizeof(int2) * nb) != cudaSuccess ||
+            cudaMalloc(&row_longest, sizeof(int)) != cudaSuccess || cudaMallocHost(&row_longest_h, sizeof(int)) != cudaSuccess)
           return H->fail(CH4_ERR_NOMEM, "row lists");
-        if (cudaMemsetAsync(row_count, 0, sizeof(int) * (nb + 1), H->stream) != cudaSuccess)
+        if (cudaMemsetAsync(row_count, 0, sizeof(int) * (nb + 1), H->stream) != cudaSuccess ||
+            cudaMemsetAsync(row_longest, 0, sizeof(int), H->stream) != cudaSuccess ||
+            cudaEventCreateWithFlags(&row_ev, cudaEventDisableTiming) != cudaSuccess)
           return H->fail(CH4_ERR_CUDA, "row lists");
-      } else if (cudaMalloc(&crng, sizeof(int2) * nhome()) != cudaSuccess ||
-          cudaMalloc(&busy, sizeof(int) * nreg * GATHER_BLOCK) != cudaSuccess ||
-          cudaMalloc(&dense, sizeof(int) * nreg * GATHER_BLOCK) != cudaSuccess ||
-          cudaMalloc(&bcount, sizeof(int) * nreg) != cudaSuccess || cudaMalloc(&boff, sizeof(int) * nreg) != cudaSuccess)
+      } else if (!home_buffers()) {
         return H->fail(CH4_ERR_NOMEM, "home-cell ranges");
+      }
     }
     if (fmoments()) {
       // A z-slab's partials are gathered with every other slab's into one z-ordered array,
@@ -1888,7 +1974,11 @@ struct Engine : EngineBase {
           }
           P.feat |= K_TWOWAY;
           if (c.resume || n_step > 1) {
+            // the slots are re-sorted after this deposit, and it is the turn to look at the lists
+            const bool look = rows_able() && np > 0 && since_reorder + 1 >= REORDER_EVERY && sorts_done++ % LOOK_EVERY == 0;
+            if (look && (st = choose_route())) return st;
             PartParams<A> Q = part_params();
+            if (look && !rows_on) Q.row_watch = row_resume(Q.segs);
             size_t bytes = cubbytes;
             if (pslab() && mig) {
               // the records of the particles next to a face go to the neighbour, theirs come in
@@ -1911,6 +2001,7 @@ struct Engine : EngineBase {
                 return st;
               }
               rows_ready = false;  // used up: a step that fails from here on is followed by a deposit from the state
+              if (look && (st = ask_longest())) return st;
               // (unless by rows, the deposit's sort already holds the slots in home-cell order)
               if (np > 0 && ++since_reorder >= REORDER_EVERY && (st = reorder_particles(by_rows() ? 1 : 0))) return st;
             }

@@ -64,6 +64,21 @@ __host__ __device__ __forceinline__ int row_edge_bin(int hx, int hy, int hz, con
 // places of a particle: one, and with edge lists a second
 __host__ __device__ __forceinline__ int row_places(const RowSegs& g) { return g.n > 1 ? 2 : 1; }
 
+// The longest list with which the deposit still goes by rows, and (row_resume) the one with which
+// it returns to them.  One warp walks a row's merged entries one after the other, while by home cells
+// every cell has a thread of its own, so rows lose once lists are long, whether the particles are
+// dense or gathered in a few rows.  us a step by home cells / by rows, FP32, by mean list (with
+// particles spread evenly the longest of a lattice is some four deviations more: 97 for 64, 135 for 96):
+//   64^3 24: 174 / 90, 64: 216 / 194, 80: 239 / 233, 128: 281 / 364;  128^3 64: 655 / 633, 96: 834 /
+//   901;  160^3 16: 506 / 426, 64: 1,021 / 1,010, 96: 1,304 / 1,422;  60x50x70 FP64 32: 203 / 126,
+//   64: 236 / 209, 96: 262 / 291.  Rows cut into segments, 512x128x64 32: 777 / 719, 48: 991 / 968;
+//   300x128x96 55: 957 / 967.
+//   Gathered in 160^3: 170,000 between two planes (longest some 600) 407 / 630, a million 763 /
+//   2,805; in 64 clusters (some 200) 548 / 494, the one case seen that the limit costs; in 256
+//   (some 60) 416 / 344.
+__host__ __device__ __forceinline__ int row_limit(const RowSegs& g) { return g.n == 1 ? 120 : 80; }
+__host__ __device__ __forceinline__ int row_resume(const RowSegs& g) { return row_limit(g) * 3 / 4; }
+
 #ifdef __CUDACC__
 
 // Deposit record and place in its list of one particle (src/lagrange_feedback.c:34-118).  The
@@ -132,8 +147,8 @@ __global__ void deposit_rows_prepare_kernel(const PartParams<A> P) {
 }
 
 // the range of every list (bins of a warp together, at a place drawn from *cursor), the counters
-// cleared for the next sub-step
-static __global__ void row_ranges_kernel(int* count, unsigned int nb, int2* list, int* cursor) {
+// cleared for the next sub-step; the longest list beyond `limit` to *longest
+static __global__ void row_ranges_kernel(int* count, unsigned int nb, int2* list, int* cursor, int limit, int* longest) {
   grid_chain();
   const unsigned int b = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
   const int c = b < nb ? count[b] : 0;
@@ -143,6 +158,8 @@ static __global__ void row_ranges_kernel(int* count, unsigned int nb, int2* list
     const int v = __shfl_up_sync(0xffffffffu, sum, d);
     if ((int)lane >= d) sum += v;
   }
+  const int most = __reduce_max_sync(0xffffffffu, c);
+  if (lane == 0 && most > limit) atomicMax(longest, most);
   int base = 0;
   if (lane == 31 && sum > 0) base = atomicAdd(cursor, sum);
   base = __shfl_sync(0xffffffffu, base, 31) + sum - c;

@@ -99,6 +99,8 @@ struct PartParams {
   int* row_count;        // [row_bins] places drawn, then the cursor that the lists' ranges are drawn from
   int2* row_list;        // [row_bins] first entry and end of every list
   int2* row_entry;       // [row_places * np] {index, slot} by list
+  int* row_longest;      // longest list seen beyond the limit
+  int row_watch;         // by home cells: note in row_longest if a list would hold more than this (0: don't look)
   double* srec;          // [nrec][np] the same by sorted position (depositing particles only)
   int* spid;             // particle index by sorted position
   int2* cell_rng;        // [(NX+1)(NY+1)(NZ+1)] {start, end} of every home cell's sorted run
@@ -1338,6 +1340,7 @@ __global__ void ghost_arrive_kernel(const PartParams<A> P, const double* from_do
 // [start, end) of every home cell in the sorted key array, and the records and
 // particle indices copied into sorted order (the gather then reads each home list
 // as one contiguous run)
+__host__ __device__ __forceinline__ int row_seg(int hx, const RowSegs& g);
 template <typename A>
 __global__ void cell_range_kernel(const PartParams<A> P, const unsigned int* key, const int* slot_of, unsigned int nh) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1347,6 +1350,12 @@ __global__ void cell_range_kernel(const PartParams<A> P, const unsigned int* key
   if (k >= nh) return;
   if (i == 0 || key[i - 1] != k) P.cell_rng[k].x = i;
   if (i == n - 1 || key[i + 1] != k) P.cell_rng[k].y = i + 1;
+  if (P.row_watch > 0 && i + P.row_watch < n) {
+    // home cells in key order: a list by rows is a run of them
+    const unsigned int k1 = key[i + P.row_watch], row = (unsigned)(P.NX + 1);
+    if (k1 < nh && k / row == k1 / row && row_seg((int)(k % row), P.segs) == row_seg((int)(k1 % row), P.segs))
+      *P.row_longest = P.row_watch + 1;  // the same value from every thread that finds one
+  }
   const int s = slot_of[i];
   P.spid[i] = P.pid[s];
   for (int f = 0; f < P.nrec; f++) P.srec[(long long)f * n + i] = P.rec[(long long)f * P.rstride + s];

@@ -19,6 +19,8 @@
 
 namespace {
 std::string g_log, g_faults, g_fail;
+int g_longest = 0;       // what the deposit reports as its longest row list
+size_t g_refused = 0;    // allocations of this size and more are refused
 bool g_pending = false;  // unfinished work on the legacy stream
 int g_streams = 0;
 
@@ -44,9 +46,14 @@ extern "C" {
 const char* fake_log() { return g_log.c_str(); }
 const char* fake_faults() { return g_faults.c_str(); }
 void fake_fail(const char* f) { g_fail = f; }
+void fake_refuse(size_t n) { g_refused = n; }
+void fake_longest(int n) { g_longest = n; }
 void fake_reset() { g_log.clear(), g_faults.clear(), g_fail.clear(); }
 
-cudaError_t cudaMalloc(void** p, size_t n) { return (*p = std::calloc(1, n ? n : 1)) ? cudaSuccess : cudaErrorMemoryAllocation; }
+cudaError_t cudaMalloc(void** p, size_t n) {
+  if (g_refused && n >= g_refused) return cudaErrorMemoryAllocation;
+  return (*p = std::calloc(1, n ? n : 1)) ? cudaSuccess : cudaErrorMemoryAllocation;
+}
 cudaError_t cudaFree(void* p) { return std::free(p), cudaSuccess; }
 cudaError_t cudaMallocHost(void** p, size_t n) { return cudaMalloc(p, n); }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return cudaMalloc(p, n); }
@@ -85,6 +92,7 @@ cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { return *ms = 1.0f, cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
 cudaError_t cudaGetDevice(int* d) { return *d = 0, cudaSuccess; }
 cudaError_t cudaGetDeviceProperties_v2(cudaDeviceProp* p, int) {
   std::memset(p, 0, sizeof *p);
@@ -154,7 +162,11 @@ using S = cudaStream_t;
   }                                                                                                                    \
   cudaError_t launch_deposit(const PartParams<A>& P, unsigned int*, int*, void* tmp, size_t&, S st, int stage) {       \
     if (P.nsort > 0) need("launch_deposit", tmp);                                                                      \
-    return launched("launch_deposit", st, "stage " + std::to_string(stage) + (P.rows_ready ? " ready" : ""));          \
+    if (P.nsort > 0 && !P.rows) need("launch_deposit", P.cell_rng), need("launch_deposit", P.srec);                    \
+    if (P.row_longest && (P.rows ? g_longest > row_limit(P.segs) : P.row_watch && g_longest > P.row_watch))            \
+      *P.row_longest = g_longest;                                                                                      \
+    return launched("launch_deposit", st, "stage " + std::to_string(stage) + (P.rows_ready ? " ready" : "") +          \
+                                              (P.nsort > 0 && P.row_count && !P.rows ? " cells" : ""));                \
   }                                                                                                                    \
   cudaError_t launch_ghosts_out(const PartParams<A>&, double* down, double* up, int, int* counts, S st) {              \
     need("launch_ghosts_out", down), need("launch_ghosts_out", counts);                                                \

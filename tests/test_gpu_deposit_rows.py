@@ -81,6 +81,51 @@ def test_cut_rows(nx, ends, n, steps):
         assert np.array_equal(got[k], v), k
 
 
+def flyers(n, size, gather):
+    """Heavy particles that keep their velocity: towards the middle, where they meet after 100
+    steps, or out of two home rows."""
+    rng = np.random.default_rng(n)
+    parts = make_particles(rng, n, *size)
+    for i, p in enumerate(parts):
+        p.tau_drag, p.beta_coeff = 1e4, 1e-9 * (1 + i % 3)
+        for a, s in zip("xyz", size):
+            v = 0.1 * (rng.random() - 0.5)
+            if gather:
+                v = (0.5 * s + 0.25 - getattr(p, a)) / 100
+            elif a != "x":
+                setattr(p, a, 2.0 + rng.random())
+            setattr(p, "v" + a, v)
+    return parts
+
+
+@pytest.mark.parametrize("gather", [False, True])
+@pytest.mark.parametrize("size", [(10, 8, 7), (260, 5, 4)])
+def test_both_routes_and_their_change(size, gather):
+    """Lists beyond the limit deposit by home cells: from the upload on where the particles are
+    gathered then, and from the second look after they have met.  530 steps hold looks at 2, 258
+    and 514.  Bit-identical to the restatement all the way."""
+    _, cfg, state = make_case("particles", seed=2, dims=size, time_dt_lagr_factor=1.0, Amp_x=1e-5, Amp_y=1e-5,
+                              Amp_z=1e-5)
+    parts = flyers(600, size, gather)
+    with ch4b200.Simulation(cfg) as sim:
+        ref = O.Restatement(cfg)
+        for s in (ref, sim):
+            s.set_pop("p", state["p"])
+            s.set_particles(parts)
+            s.initialize()
+        for steps in (5, 525):
+            ref.step(steps)
+            sim.step(steps)
+            want = ref.get_pop("p")
+            assert np.isfinite(want).all()
+            assert np.array_equal(sim.get_pop("p"), want)
+            assert np.abs(sim.force() - ref.force()).max() == 0
+            got, want = (O.particles_as_dict(s.get_particles(len(parts))) for s in (sim, ref))
+            for k, v in want.items():
+                assert np.array_equal(got[k], v), k
+        ref.close()
+
+
 @pytest.mark.parametrize("name", ["segments", "dense"])
 def test_rows_f32_reproducible(name):
     c = CASES[name]

@@ -28,6 +28,7 @@ def fakes(tmp_path_factory):
                     os.path.join(HERE, "host_fakes.cpp"), "-o", so], check=True)
     L = C.CDLL(so)
     L.fake_log.restype = L.fake_faults.restype = C.c_char_p
+    L.fake_refuse.argtypes = [C.c_size_t]
     return L
 
 
@@ -186,3 +187,71 @@ def test_u_of_the_les_after_a_failed_step(handle, fakes):
         counts.append(les.log().count("launch_hydro"))
     assert counts == [2, 1, 1, 2, 1]
     les.close()
+
+
+LOOK = 256  # steps between two looks at the lists: every 16th re-sort
+
+
+def routes(h):
+    """Steps that deposited by home cells, among the deposits since the last call."""
+    return ["cells" in x for x in h.log() if "deposit" in x]
+
+
+def crowd(parts, cfg, rows):
+    """The particles, all depositing, in one home row or spread."""
+    parts = type(parts)(*parts)
+    for i, p in enumerate(parts):
+        p.tau_drag, p.beta_coeff = 1.0, 1.0
+        p.y, p.z = (2.0, 2.0) if rows else (i % cfg.NY + 0.5, i // cfg.NY % cfg.NZ + 0.5)
+    return parts
+
+
+def test_deposit_route_follows_the_longest_list(handle, fakes):
+    """At ch4_set_particles by the positions, then at every look by the figure of the one before."""
+    fakes.fake_longest(0)
+    h, state = handle("particles")
+    h.set_particles(crowd(state["part"], h.cfg, True))  # 300 particles in one row
+    h.initialize()
+    assert h.step(2 + LOOK - 1) == 0
+    assert routes(h) == [True] * LOOK  # the first step deposits nothing
+    assert h.step(1) == 0  # the first look found no long list
+    assert routes(h) == [False]
+    fakes.fake_longest(91)
+    assert h.step(LOOK) == 0  # longer than to return to rows, not than to leave them
+    assert routes(h) == [False] * LOOK
+    fakes.fake_longest(121)
+    assert h.step(LOOK) == 0
+    assert routes(h) == [False] * LOOK
+    fakes.fake_longest(91)
+    assert h.step(LOOK) == 0
+    assert routes(h) == [False] * (LOOK - 1) + [True]
+    assert h.step(LOOK) == 0
+    assert routes(h) == [True] * LOOK
+    h.set_particles(crowd(state["part"], h.cfg, False))
+    assert h.step(1) == 0
+    assert routes(h) == [False]
+    h.set_particles((abi.Particle * 0)())
+    assert h.step(2) == 0
+    h.set_particles(crowd(state["part"], h.cfg, True))
+    assert h.step(1) == 0
+    assert routes(h) == [False, False, True]
+    fakes.fake_longest(0)
+
+
+def test_deposit_stays_by_rows_without_memory(handle, fakes):
+    """Where the buffers of the home cells are refused the deposit goes by rows as before, and
+    takes them when there is room."""
+    h, state = handle("particles")
+    parts = crowd(state["part"], h.cfg, True)
+    h.set_particles(crowd(state["part"], h.cfg, False))
+    h.initialize()
+    h.log()
+    for refused in (1, 8 * 9 * len(parts)):  # the first buffer, and the last
+        fakes.fake_refuse(refused)
+        h.set_particles(parts)
+        assert h.step(2) == 0
+        fakes.fake_refuse(0)
+        assert not any(routes(h))
+    h.set_particles(parts)
+    assert h.step(1) == 0
+    assert routes(h) == [True]

@@ -1914,12 +1914,11 @@ struct Engine : EngineBase {
     if (!uhalo && cudaMalloc(&uhalo, 4 * part * sizeof(A)) != cudaSuccess) return H->fail(CH4_ERR_NOMEM, "u halo");
     A *send_down = uhalo, *send_up = uhalo + part, *from_up = uhalo + 2 * part, *from_down = uhalo + 3 * part;
     HaloCopy hc{};
-    hc.src[hc.n] = ules;
-    hc.dst[hc.n] = send_down;
-    hc.bytes[hc.n++] = part * sizeof(A);
-    hc.src[hc.n] = ules + (size_t)(c.NZ - 1) * part;
-    hc.dst[hc.n] = send_up;
-    hc.bytes[hc.n++] = part * sizeof(A);
+    hc.src[0] = reinterpret_cast<const uint32_t*>(ules);
+    hc.src[1] = reinterpret_cast<const uint32_t*>(ules + (size_t)(c.NZ - 1) * part);
+    hc.dst[0] = reinterpret_cast<uint32_t*>(send_down);
+    hc.dst[1] = reinterpret_cast<uint32_t*>(send_up);
+    hc.words = part * sizeof(A) / sizeof(uint32_t);
     if ((st = H->cuda(launch_halo_copy(hc, H->stream), "u faces"))) return st;
     if (H->exchange(send_down, send_up, from_up, from_down, part * sizeof(A), H->stream, H->exchange_user) != 0)
       return H->fail(CH4_ERR_CUDA, "the exchange of the slabs' u planes failed");

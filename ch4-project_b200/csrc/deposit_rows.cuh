@@ -34,7 +34,7 @@ constexpr int ROW_SEG = 256;    // cells of a row that one warp owns, at most
 constexpr int ROW_CUT_SHIFT = 7, ROW_CUT = 1 << ROW_CUT_SHIFT;  // cells of a segment of a longer row
 constexpr int ROW_CHUNK = 64;   // merged entries in shared memory at a time
 constexpr int ROW_WARPS = 4;    // warps per block
-constexpr int ROW_REC = 10;     // doubles of a record: fac*fp (3), dxm dxp dym dyp dzm dzp, {hx, index}
+constexpr int ROW_REC = 10;     // doubles of a record: fac*fp (3), dxm dxp dym dyp dzm dzp, hx (as int)
 
 // the segments of a row of NX cells: all of `len` cells but for the last; the last home cell (hx =
 // NX) belongs to the last segment
@@ -95,7 +95,6 @@ __device__ __forceinline__ void deposit_rows_emit(const PartParams<A>& P, int ip
   const bool inside = wrapped_position(P, x, y, z, px, py, pz);
   make_stencil(px, py, pz, t);
   const double fac = pf[PF_VOL * np + ip];
-  const int o = P.pid[ip];
   const bool live = inside && (fac > 0.0) && beta != 0.0;
   const int hx = t.im + 1, hy = t.jm + 1, hz = t.km + 1;
   if (P.segs.n > 1) {
@@ -131,7 +130,7 @@ __device__ __forceinline__ void deposit_rows_emit(const PartParams<A>& P, int ip
   r[1] = make_double2(f[2], t.dxm);
   r[2] = make_double2(t.dxp, t.dym);
   r[3] = make_double2(t.dyp, t.dzm);
-  r[4] = make_double2(t.dzp, __hiloint2double(o, hx));
+  r[4] = make_double2(t.dzp, __hiloint2double(0, hx));
 }
 
 // the same from the state (a resumed run's first deposit; random re-entry, which moves

@@ -6,13 +6,15 @@
 
 namespace ch4 {
 
-// Up to two sets: three 256-thread blocks per SM (80 registers; three sets would spill): 48 lattices of 64x64 .. 512x256, FP32 fluid and
-// temperature, 94.4 us a step against 97.3 at the 101 registers it takes unbounded
+// Launched and captured the ordinary way (chained graph nodes measured the same), so it begins
+// without grid_chain() and reads its list through the read-only path.
+// Up to two sets: three 256-thread blocks per SM (80 registers, at most 8 bytes spilled;
+// three sets would spill more): 48 lattices of 64x64 .. 512x256, FP32 fluid and temperature, 94.4 us
+// a step against 97.3 at the 101 registers it takes unbounded
 template <typename S, typename A, bool THERM, bool SCAL>
 __global__ void __launch_bounds__(256, THERM && SCAL ? 2 : 3) ensemble_step_kernel(const StepParams<A>* __restrict__ params,
                                                             const EnsTile* __restrict__ tiles, int ntiles,
                                                             int* counter) {
-  grid_chain();
   __shared__ StepParams<A> sp;
   __shared__ int tile_id;
   constexpr int WORDS = (int)(sizeof(StepParams<A>) / sizeof(int));

@@ -221,11 +221,14 @@ __device__ __forceinline__ S* pop_at(void* set, uint32_t bstride, long long idx)
   return const_cast<S*>(pop_at<S>(const_cast<const void*>(set), bstride, idx));
 }
 
-// Programmatic dependent launch: every kernel of the step begins here.  Launched with the
-// attribute (launch_chained) it may be resident before the kernel ahead of it in the stream has
-// ended; it waits for that kernel's end and its writes, then lets the next one come.  What one
-// kernel of the chain writes the next one reads with plain loads: the read-only path promises
-// nothing for data written after a kernel's launch.  The gap between two dependent kernels was
+// Programmatic dependent launch: a kernel launched with the attribute (launch_chained: the step, the
+// u^n pass, the SISM mean, the row lists and the deposit by rows, the re-sort's permutation) begins
+// here.  It may be resident before the kernel ahead of it in the stream has ended; it waits for
+// that kernel's end and its writes, then lets the next one come.  What one kernel of the chain
+// writes the next one reads with plain loads: the read-only path promises nothing for data written
+// after a kernel's launch.  The particle sub-step reads through it and is launched the ordinary
+// way; it begins here only to let the next one come.  The force sums, the home-cell deposit and
+// the sorts are outside the chain.  The gap between two dependent kernels was
 // 2 us: us a step, Kolmogorov 32^3 FP32 4.7 -> 3.4, 64^3 FP32 10.3 -> 6.9, 64^3 FP64 14.6 ->
 // 12.8, Rayleigh-Benard 32^3 FP32 10.3 -> 7.8, LES with tracers 96^3 62 -> 55.
 __device__ __forceinline__ void grid_chain() {

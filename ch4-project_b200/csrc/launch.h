@@ -79,13 +79,11 @@ inline size_t halo_word(const void* down, const void* up, size_t bytes) {
   return bytes > 1 ? bytes : 0;
 }
 cudaError_t launch_halo_faces(const HaloFacesArgs& a, size_t bytes, cudaStream_t st);
-// copies of up to 30 device regions (the u faces of a z-slab), in 4-byte words when every
-// region's size and addresses allow it, else in 2-byte words
+// copies of two device regions (the u faces of a z-slab) of `words` 4-byte words
 struct HaloCopy {
-  const void* src[30];
-  void* dst[30];
-  size_t bytes[30];
-  int n;
+  const uint32_t* src[2];
+  uint32_t* dst[2];
+  size_t words;
 };
 cudaError_t launch_halo_copy(const HaloCopy& H, cudaStream_t st);
 

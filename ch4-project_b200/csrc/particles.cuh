@@ -834,7 +834,7 @@ __device__ __forceinline__ void deposit_rows_emit(const PartParams<A>& P, int ip
 // FP32: four blocks of 128 per SM (<= 128 registers); FP64 keeps twice the registers
 template <typename A, bool ORIENT, bool HALO, int NF>
 __global__ void __launch_bounds__(128, sizeof(A) == 8 ? 2 : 4) particle_substep_kernel(const PartParams<A> P) {
-  grid_chain();
+  grid_chain();  // for the kernel after it: this one reads the velocities through the read-only path
   const int ip = blockIdx.x * blockDim.x + threadIdx.x;
   if (ip >= P.np) return;
   double* pf = P.pf;
